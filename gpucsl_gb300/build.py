@@ -20,7 +20,7 @@ BUILD = PKG / "_build"
 LIB = PKG / "libgpucsl_gb300.so"
 BUILD_DEBUG = PKG / "_build_debug"
 LIB_DEBUG = PKG / "libgpucsl_gb300_debug.so"
-SOURCES = ["gauss.cu", "capi.cu", "corr.cu", "discrete.cu", "noalloc.cu", "tc_gemm.cu", "corr_tc.cu", "gauss_batch.cu", "orient.cu", "encode.cu"]
+SOURCES = ["gauss.cu", "capi.cu", "corr.cu", "discrete.cu", "disc_bits.cu", "noalloc.cu", "tc_gemm.cu", "corr_tc.cu", "gauss_batch.cu", "orient.cu", "encode.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr"]
 

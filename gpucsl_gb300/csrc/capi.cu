@@ -26,7 +26,6 @@ cudaError_t launch_compact(const uint16_t *G, int p, int *adj, int *up, DevState
 cudaError_t launch_scan_int(const int *cnt, int p, long long *prefix, DevState *st, cudaStream_t s);
 cudaError_t launch_recompact(const uint16_t *G, int p, int *adj, int *up, DevState *st, int level, int2 *elist,
                              cudaStream_t s);
-cudaError_t launch_scan_ll(const long long *cnt, int p, long long *prefix, DevState *st, cudaStream_t s);
 cudaError_t launch_gauss_level(int L, const double *C, int p, const int *adj, const int *up, const int2 *elist,
                                const long long *prefix, double tau, bool tau_valid, uint16_t *G, double *zmin,
                                double *r2min, int *sep_dense, int max_level, int *rec_pool, long long rec_cap,
@@ -54,13 +53,19 @@ int disc_table_cap(int device);
 void disc_level_caps(int cap_full, int max_dim, int L, int &table_cap, int &part_cap);
 cudaError_t launch_disc_tests(const DiscLevelArgs &A, int num_sms, cudaStream_t s);
 cudaError_t launch_disc_validate(const uint8_t *data, long long ld, long long n, int p, const uint8_t *dims,
-                                 DevState *st, int num_sms, cudaStream_t s);
-cudaError_t launch_disc_weights(const int *adj, int p, int L, long long *w, DevState *st, cudaStream_t s);
+                                 double *lg, DevState *st, int num_sms, cudaStream_t s);
+cudaError_t launch_disc_plan(const int *adj, int p, int L, int group, const uint8_t *dims, long long *w,
+                             long long *prefix, long long *tasks, int *rows, DevState *st, cudaStream_t s);
+bool disc_bits_ok(long long n, int p, int max_dim);
+size_t disc_bits_words(long long n, int p, int max_dim);
+int disc_bits_group(int max_dim);
+size_t disc_lgam_doubles();
+cudaError_t launch_disc_bits_level0(const DiscBits &b, const DiscLevelArgs &A, int num_sms, cudaStream_t s);
+cudaError_t launch_disc_bits_level1(const DiscBits &b, const DiscLevelArgs &A, const long long *tasks,
+                                    const int *rows, int num_sms, cudaStream_t s);
 cudaError_t launch_disc_finalize(const int *adj, int p, int L, uint16_t *G, unsigned long long *win, int *sep,
                                  int max_level, int *rec, long long rec_cap, DevState *st, int num_sms,
                                  cudaStream_t s);
-cudaError_t launch_disc_level_stats(const long long *prefix, const int *adj, int p, int L, DevState *st,
-                                    cudaStream_t s);
 cudaError_t launch_pmax_finish(double *pmax, int p, int num_sms, cudaStream_t s);
 cudaError_t launch_disc_table(const uint8_t *data, long long ld, long long n, const uint8_t *dims, int vi, int vj,
                               const int *S, int L, int table_cap, uint32_t *counts, long long counts_cap, double *out2,
@@ -503,21 +508,91 @@ GaussWs carve_gauss(void *ws, size_t cap, int p) {
 struct DiscWs {
     DevState *st;
     int *adj;
-    long long *weights, *prefix;
+    long long *weights, *prefix, *tasks;
+    int *rows;
     unsigned long long *win;
+    DiscBits bits;  // the bit-plane path's buffers when the shape takes it (planes != nullptr)
     size_t bytes;
 };
 
-DiscWs carve_disc(void *ws, size_t cap, int p) {
+DiscWs carve_disc(void *ws, size_t cap, int p, long long n, int max_dim) {
     Carver c(ws, cap);
     DiscWs w;
     w.st = c.take<DevState>(1);
     w.adj = c.take<int>((size_t)p * p);
     w.weights = c.take<long long>((size_t)p);
     w.prefix = c.take<long long>((size_t)p + 1);
+    w.tasks = c.take<long long>((size_t)p + 1);
+    w.rows = c.take<int>((size_t)p);
     w.win = c.take<unsigned long long>((size_t)p * p);
+    std::memset(&w.bits, 0, sizeof(w.bits));
+    w.bits.max_dim = max_dim;
+    w.bits.lg = c.take<double>(host::disc_lgam_doubles());
+    if (host::disc_bits_ok(n, p, max_dim)) {
+        const size_t pl = (size_t)p * (max_dim - 1), va = (size_t)p * max_dim;
+        w.bits.planes = c.take<uint32_t>(host::disc_bits_words(n, p, max_dim));
+        w.bits.counts = c.take<uint32_t>(pl * pl);
+        w.bits.full = c.take<uint32_t>(va * va);
+        w.bits.inv = c.take<double>(va * va);
+        w.bits.card = c.take<uint8_t>((size_t)p);
+        w.bits.off = c.take<int>((size_t)p + 1);
+        w.bits.foff = c.take<int>((size_t)p + 1);
+    }
     w.bytes = c.off;
     return w;
+}
+
+// One discrete solve; with bits, levels 0 and 1 run on bit planes.
+int disc_solve(DiscLevelArgs A, const DiscWs &w, bool bits, int max_dim, int max_level, int *sepsets, int *rec_pool,
+               long long rec_cap, gcsl_stats *stats, cudaStream_t s) {
+    const int sms = device_sms(), p = A.p;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const int cap = host::disc_table_cap(dev);
+    if ((long long)max_dim * max_dim > cap) return GCSL_ERR_UNSUPPORTED;
+    cudaError_t e = cudaMemsetAsync(w.st, 0, sizeof(DevState), s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(w.win, 0xff, sizeof(unsigned long long) * (size_t)p * p, s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(A.pmax, 0, sizeof(double) * (size_t)p * p, s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(A.G, 0, sizeof(uint16_t) * (size_t)p * p, s);
+    if (e != cudaSuccess) return GCSL_ERR_DEVICE;
+    A.order = host::work_order_seed();
+    host::disc_level_caps(cap, max_dim, 0, A.table_cap, A.part_cap);
+    if (bits) {
+        if (host::launch_disc_bits_level0(w.bits, A, sms, s) != cudaSuccess) return GCSL_ERR_DEVICE;
+    } else {
+        // codes in range once per solve; the test kernels skip the per-sample checks then
+        if (host::launch_disc_validate(A.data, A.ld, A.n, p, A.dims, w.bits.lg, w.st, sms, s) != cudaSuccess)
+            return GCSL_ERR_DEVICE;
+        if (host::launch_disc_tests(A, sms, s) != cudaSuccess) return GCSL_ERR_DEVICE;
+    }
+    HostCtl *hc = host_ctl();
+    if (!hc) return GCSL_ERR_DEVICE;
+    auto disc_level = [&](int level) -> cudaError_t {
+        const bool planes = bits && level == 1;
+        cudaError_t e2 = host::launch_compact(A.G, p, w.adj, nullptr, w.st, level, nullptr, s);
+        if (e2 == cudaSuccess)
+            e2 = host::launch_disc_plan(w.adj, p, level, planes ? host::disc_bits_group(max_dim) : 0, A.dims,
+                                        w.weights, w.prefix, w.tasks, w.rows, w.st, s);
+        DiscLevelArgs B = A;
+        B.level = level;
+        host::disc_level_caps(cap, max_dim, level, B.table_cap, B.part_cap);
+        if (e2 == cudaSuccess)
+            e2 = planes ? host::launch_disc_bits_level1(w.bits, B, w.tasks, w.rows, sms, s) : host::launch_disc_tests(B, sms, s);
+        if (e2 == cudaSuccess)
+            e2 = host::launch_disc_finalize(w.adj, p, level, A.G, w.win, sepsets, max_level, rec_pool, rec_cap, w.st,
+                                            sms, s);
+        return e2;
+    };
+    const int rc = run_levels(max_level, w.st, s, hc->words, [&](int a, int b) -> cudaError_t {
+        for (int level = a; level <= b; ++level) {
+            const cudaError_t e2 = disc_level(level);
+            if (e2 != cudaSuccess) return e2;
+        }
+        return cudaSuccess;
+    });
+    if (rc != GCSL_OK) return rc;
+    if (host::launch_pmax_finish(A.pmax, p, sms, s) != cudaSuccess) return GCSL_ERR_DEVICE;
+    return finish_stats(w.st, stats, s, true, p);
 }
 
 }  // namespace
@@ -759,10 +834,8 @@ int gcsl_gauss_skeleton(const double *C, int32_t p, int64_t n_obs, const double 
 }
 
 size_t gcsl_disc_workspace_bytes(int32_t p, int64_t n, int32_t max_level, int32_t max_dim) {
-    (void)n;
     (void)max_level;
-    (void)max_dim;
-    return carve_disc(nullptr, 0, p).bytes;
+    return carve_disc(nullptr, 0, p, n, max_dim).bytes;
 }
 
 int gcsl_disc_skeleton(const uint8_t *data, int64_t ld, int64_t n, int32_t p, const uint8_t *dims, int32_t max_dim,
@@ -773,51 +846,15 @@ int gcsl_disc_skeleton(const uint8_t *data, int64_t ld, int64_t n, int32_t p, co
         max_dim < 1 || max_dim > 255 || reinterpret_cast<uintptr_t>(data) % 16 != 0)
         return GCSL_ERR_INVALID_ARG;
     if (rec_pool == nullptr) rec_cap = 0;
-    DiscWs w = carve_disc(workspace, workspace_bytes, p);
+    const DiscWs w = carve_disc(workspace, workspace_bytes, p, n, max_dim);
     if (!workspace || w.bytes > workspace_bytes) return GCSL_ERR_WORKSPACE;
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const int sms = device_sms();
-    int dev = 0;
-    cudaGetDevice(&dev);
-    const int cap = host::disc_table_cap(dev);
-    if ((long long)max_dim * max_dim > cap) return GCSL_ERR_UNSUPPORTED;
-    cudaError_t e = cudaMemsetAsync(w.st, 0, sizeof(DevState), s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(w.win, 0xff, sizeof(unsigned long long) * (size_t)p * p, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(pmax, 0, sizeof(double) * (size_t)p * p, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(G, 0, sizeof(uint16_t) * (size_t)p * p, s);
-    if (e != cudaSuccess) return GCSL_ERR_DEVICE;
-    DiscLevelArgs A{data, ld, n, p, dims, alpha, 0, w.adj, w.prefix, G, pmax, w.win, cap, 1024, w.st};
-    A.order = host::work_order_seed();
-    host::disc_level_caps(cap, max_dim, 0, A.table_cap, A.part_cap);
-    // codes in range once per solve; the test kernels skip the per-sample checks then
-    if (host::launch_disc_validate(data, ld, n, p, dims, w.st, sms, s) != cudaSuccess) return GCSL_ERR_DEVICE;
-    if (host::launch_disc_tests(A, sms, s) != cudaSuccess) return GCSL_ERR_DEVICE;
-    HostCtl *hc = host_ctl();
-    if (!hc) return GCSL_ERR_DEVICE;
-    auto disc_level = [&](int level) -> cudaError_t {
-        cudaError_t e2 = host::launch_compact(G, p, w.adj, nullptr, w.st, level, nullptr, s);
-        if (e2 == cudaSuccess) e2 = host::launch_disc_weights(w.adj, p, level, w.weights, w.st, s);
-        if (e2 == cudaSuccess) e2 = host::launch_scan_ll(w.weights, p, w.prefix, w.st, s);
-        if (e2 == cudaSuccess) e2 = host::launch_disc_level_stats(w.prefix, w.adj, p, level, w.st, s);
-        DiscLevelArgs B = A;
-        B.level = level;
-        host::disc_level_caps(cap, max_dim, level, B.table_cap, B.part_cap);
-        if (e2 == cudaSuccess) e2 = host::launch_disc_tests(B, sms, s);
-        if (e2 == cudaSuccess)
-            e2 = host::launch_disc_finalize(w.adj, p, level, G, w.win, sepsets, max_level, rec_pool, rec_cap, w.st,
-                                            sms, s);
-        return e2;
-    };
-    int rc = run_levels(max_level, w.st, s, hc->words, [&](int a, int b) -> cudaError_t {
-        for (int level = a; level <= b; ++level) {
-            const cudaError_t e2 = disc_level(level);
-            if (e2 != cudaSuccess) return e2;
-        }
-        return cudaSuccess;
-    });
-    if (rc != GCSL_OK) return rc;
-    if (host::launch_pmax_finish(pmax, p, sms, s) != cudaSuccess) return GCSL_ERR_DEVICE;
-    return finish_stats(w.st, stats, s, true, p);
+    DiscLevelArgs A{data, ld, n, p, dims, alpha, 0, w.adj, w.prefix, G, pmax, w.win, 0, 1024, w.st, w.bits.lg};
+    int rc = disc_solve(A, w, w.bits.planes != nullptr, max_dim, max_level, sepsets, rec_pool, rec_cap, stats,
+                        static_cast<cudaStream_t>(stream));
+    if (rc == DISC_STATUS_WIDE)  // a cardinality above max_dim: the general path takes it if its tables fit
+        rc = disc_solve(A, w, false, max_dim, max_level, sepsets, rec_pool, rec_cap, stats,
+                        static_cast<cudaStream_t>(stream));
+    return rc;
 }
 
 int gcsl_compact(const uint16_t *G, int32_t p, int32_t *adj, void *stream) {

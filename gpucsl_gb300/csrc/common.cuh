@@ -199,8 +199,24 @@ struct DiscLevelArgs {
     int table_cap;            // counters of shared memory for the table and its replicas
     int part_cap;             // strata of the per-stratum statistic buffer (after the table)
     DevState *st;
+    const double *lg;         // ln Gamma tables of the p-value series
     unsigned long long order = 0;  // work order of the debug build (0: launch order)
 };
+
+// Buffers of the bit-plane path of discrete levels 0 and 1 (disc_bits.cu), sized for p
+// variables of at most max_dim values.
+struct DiscBits {
+    int max_dim;
+    uint32_t *planes;  // one bit plane per value but the last of every variable
+    uint32_t *counts;  // counts of all pairs of planes
+    uint32_t *full;    // counts of all pairs of values
+    double *inv;       // their reciprocals (0 for an empty pair)
+    uint8_t *card;     // cardinalities, at most max_dim
+    int *off, *foff;   // planes / values before each variable
+    double *lg;        // ln Gamma tables
+};
+// Status inside a solve (never returned): a cardinality above max_dim.
+constexpr int DISC_STATUS_WIDE = 1000;
 
 __device__ __forceinline__ void set_status(DevState *st, int code) { atomicCAS(&st->status, 0, code); }
 

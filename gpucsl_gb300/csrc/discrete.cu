@@ -2,8 +2,11 @@
 //
 //   tests          disc_test_kernel      (reference: gpucsl/pc/cuda/discrete_ci.cu:37-246,
 //                                         helpers/discrete_helpers.cu:25-186)
-//   p-value        pchisq_dev            (reference: helpers/math_helpers.cu:54-175)
+//   p-value        disc_stat.cuh         (reference: helpers/math_helpers.cu:54-175)
 //   write-back     disc_finalize_kernel  (reference: helpers/graph_helpers.cu:81-101)
+//
+// Levels 0 and 1 of tables of up to 16 values per variable run on bit planes (disc_bits.cu);
+// the kernels here take the other levels and wider tables.
 //
 // One CTA evaluates one test at a time (grid-stride over the level's flattened test
 // list): the l+2 uint8 columns are streamed with 16-byte loads and counted into a
@@ -16,135 +19,12 @@
 // As in the reference every rank of every direction is tested (discrete_ci.cu:221-244
 // has no effective early exit) and pmax folds all of them.  The removing test with the
 // smallest key (rank, dir) is the canonical remover; its set becomes the sepset.
-#include "common.cuh"
+#include <algorithm>
+
+#include "disc_stat.cuh"
+#include "gauss_dev.cuh"  // block_scan_rows
 
 namespace gcsl {
-
-// ---------------------------------------------------------------- p-value
-// Ibbetson (CACM Alg. 209) normal tail as coded by Perlman; the polynomial
-// coefficients are those of the published algorithm.
-__device__ double poz_dev(double z) {
-    double x;
-    if (z == 0.0) {
-        x = 0.0;
-    } else {
-        double y = 0.5 * fabs(z);
-        if (y >= 3.0) {
-            x = 1.0;
-        } else if (y < 1.0) {
-            const double w = y * y;
-            double t = 0.000124818987;
-            t = __dadd_rn(__dmul_rn(t, w), -0.001075204047);
-            t = __dadd_rn(__dmul_rn(t, w), 0.005198775019);
-            t = __dadd_rn(__dmul_rn(t, w), -0.019198292004);
-            t = __dadd_rn(__dmul_rn(t, w), 0.059054035642);
-            t = __dadd_rn(__dmul_rn(t, w), -0.151968751364);
-            t = __dadd_rn(__dmul_rn(t, w), 0.319152932694);
-            t = __dadd_rn(__dmul_rn(t, w), -0.531923007300);
-            t = __dadd_rn(__dmul_rn(t, w), 0.797884560593);
-            x = __dmul_rn(__dmul_rn(t, y), 2.0);
-        } else {
-            y -= 2.0;
-            double t = -0.000045255659;
-            t = __dadd_rn(__dmul_rn(t, y), 0.000152529290);
-            t = __dadd_rn(__dmul_rn(t, y), -0.000019538132);
-            t = __dadd_rn(__dmul_rn(t, y), -0.000676904986);
-            t = __dadd_rn(__dmul_rn(t, y), 0.001390604284);
-            t = __dadd_rn(__dmul_rn(t, y), -0.000794620820);
-            t = __dadd_rn(__dmul_rn(t, y), -0.002034254874);
-            t = __dadd_rn(__dmul_rn(t, y), 0.006549791214);
-            t = __dadd_rn(__dmul_rn(t, y), -0.010557625006);
-            t = __dadd_rn(__dmul_rn(t, y), 0.011630447319);
-            t = __dadd_rn(__dmul_rn(t, y), -0.009279453341);
-            t = __dadd_rn(__dmul_rn(t, y), 0.005353579108);
-            t = __dadd_rn(__dmul_rn(t, y), -0.002141268741);
-            t = __dadd_rn(__dmul_rn(t, y), 0.000535310849);
-            x = __dadd_rn(__dmul_rn(t, y), 0.999936657524);
-        }
-    }
-    return z > 0.0 ? ((x + 1.0) * 0.5) : ((1.0 - x) * 0.5);
-}
-
-__device__ __forceinline__ double ex_dev(double x) { return (x < -20.0) ? 0.0 : exp(x); }
-
-// Upper tail of chi^2 (Hill & Pike, CACM Alg. 299, with the 1985 rounding remark, in
-// Perlman's formulation): the finite series of the even / odd df cases.
-__device__ double pchisq_dev(double x, long long df) {
-    if (x <= 0.0 || df < 1) return 1.0;
-    const double a = 0.5 * x;
-    const bool even = (df & 1) == 0;
-    const double y = (df > 1) ? ex_dev(-a) : 0.0;
-    double s = even ? y : 2.0 * poz_dev(-sqrt(x));
-    if (df <= 2) return s;
-    const double half = 0.5 * ((double)df - 1.0);
-    double z = even ? 1.0 : 0.5;
-    if (a > 20.0) {
-        double e = even ? 0.0 : 0.5723649429247000870717135;
-        const double c = log(a);
-        while (z <= half) {
-            e = __dadd_rn(log(z), e);
-            s = __dadd_rn(s, ex_dev(__dsub_rn(__dsub_rn(__dmul_rn(c, z), a), e)));
-            z += 1.0;
-        }
-        return s;
-    }
-    double e = even ? 1.0 : 0.5641895835477562869480795 / sqrt(a);
-    double c = 0.0;
-    while (z <= half) {
-        e = __dmul_rn(e, a / z);
-        c = __dadd_rn(c, e);
-        z += 1.0;
-    }
-    return __dadd_rn(__dmul_rn(c, y), s);
-}
-
-// pchisq_dev by the 32 lanes of one warp, with the same result bit for bit: the
-// quotients a / z (or logarithms log z) of the series are independent and computed one
-// per lane, and the recurrence and the sums run in the same order on every lane.  On a
-// GPU whose FP64 pipe is 1/64 of its FP32 pipe this takes the divisions off the serial
-// path.  All lanes of the warp must call it; every lane returns the value.
-__device__ double pchisq_warp(double x, long long df) {
-    const int lane = threadIdx.x & 31;
-    if (x <= 0.0 || df < 1) return 1.0;
-    const double a = 0.5 * x;
-    const bool even = (df & 1) == 0;
-    const double y = (df > 1) ? ex_dev(-a) : 0.0;
-    double s = even ? y : 2.0 * poz_dev(-sqrt(x));
-    if (df <= 2) return s;
-    const double half = 0.5 * ((double)df - 1.0);
-    const double z0 = even ? 1.0 : 0.5;
-    const long long K = (long long)floor(half - z0) + 1;  // iterations z = z0, z0 + 1, .. <= half
-    if (a > 20.0) {
-        double e = even ? 0.0 : 0.5723649429247000870717135;
-        const double c = log(a);
-        for (long long k0 = 0; k0 < K; k0 += 32) {
-            const long long k = k0 + lane;
-            const double z = z0 + (double)k;
-            const double lz = k < K ? log(z) : 0.0;
-            double ek = 0.0;
-            const int m = (int)(K - k0 < 32 ? K - k0 : 32);
-            for (int q = 0; q < m; ++q) {
-                e = __dadd_rn(__shfl_sync(GCSL_FULL_MASK, lz, q), e);
-                if (lane == q) ek = e;
-            }
-            const double term = k < K ? ex_dev(__dsub_rn(__dsub_rn(__dmul_rn(c, z), a), ek)) : 0.0;
-            for (int q = 0; q < m; ++q) s = __dadd_rn(s, __shfl_sync(GCSL_FULL_MASK, term, q));
-        }
-        return s;
-    }
-    double e = even ? 1.0 : 0.5641895835477562869480795 / sqrt(a);
-    double c = 0.0;
-    for (long long k0 = 0; k0 < K; k0 += 32) {
-        const long long k = k0 + lane;
-        const double q_k = k < K ? a / (z0 + (double)k) : 0.0;
-        const int m = (int)(K - k0 < 32 ? K - k0 : 32);
-        for (int q = 0; q < m; ++q) {
-            e = __dmul_rn(e, __shfl_sync(GCSL_FULL_MASK, q_k, q));
-            c = __dadd_rn(c, e);
-        }
-    }
-    return __dadd_rn(__dmul_rn(c, y), s);
-}
 
 // ------------------------------------------------------------ test kernel
 
@@ -295,63 +175,90 @@ __device__ double stratum_chi2(const uint32_t *Ts, int di, int dj) {
     return part;
 }
 
-// stratum_chi2 by the 32 lanes of one warp (di, dj <= 32), bit for bit: lane a / b holds
-// the row / column sums, every lane one cell's term (its two divisions), and the terms
-// are added in (a, b) order as in stratum_chi2.  The sum is meaningful in every lane.
-__device__ double stratum_chi2_warp(const uint32_t *Ts, int di, int dj) {
-    const int lane = threadIdx.x & 31;
-    uint32_t ma = 0, mb = 0;
-    if (lane < di)
-        for (int b = 0; b < dj; ++b) ma += Ts[lane * dj + b];
-    if (lane < dj)
-        for (int a = 0; a < di; ++a) mb += Ts[a * dj + lane];
-    uint32_t mt = lane < di ? ma : 0u;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mt += __shfl_xor_sync(GCSL_FULL_MASK, mt, o);
-    if (mt == 0) return 0.0;
-    double part = 0.0;
-    const int cells = di * dj;
-    for (int k0 = 0; k0 < cells; k0 += 32) {
-        const int k = k0 + lane;
-        const int a = k < cells ? k / dj : 0, b = k < cells ? k - (k / dj) * dj : 0;
-        const uint32_t mak = __shfl_sync(GCSL_FULL_MASK, ma, a), mbk = __shfl_sync(GCSL_FULL_MASK, mb, b);
-        double term = 0.0;
-        bool use = false;
-        if (k < cells) {
-            const double e = __ddiv_rn(__dmul_rn((double)mak, (double)mbk), (double)mt);
-            if (e != 0.0) {
-                const double d = __dsub_rn((double)Ts[k], e);
-                term = __ddiv_rn(__dmul_rn(d, d), e);
-                use = true;
-            }
-        }
-        const unsigned um = __ballot_sync(GCSL_FULL_MASK, use);
-        const int m = cells - k0 < 32 ? cells - k0 : 32;
-        for (int q = 0; q < m; ++q) {
-            const double t = __shfl_sync(GCSL_FULL_MASK, term, q);
-            if ((um >> q) & 1u) part = __dadd_rn(part, t);
-        }
-    }
-    return part;
-}
-
-// Statistic of the counted table: strata in parallel (a warp per stratum), then added in
-// ascending s by thread 0 (the return value is meaningful in thread 0 only).
-__device__ double table_chi2(const uint32_t *sm_tab, int dim_s, int di, int dj, double *s_part) {
-    if (di <= 32 && dj <= 32) {
-        const int warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-        for (int s = warp; s < dim_s; s += nwarps) {
-            const double part = stratum_chi2_warp(sm_tab + (size_t)s * di * dj, di, dj);
-            if ((threadIdx.x & 31) == 0) s_part[s] = part;
-        }
-    } else {
-        for (int s = threadIdx.x; s < dim_s; s += blockDim.x)
-            s_part[s] = stratum_chi2(sm_tab + (size_t)s * di * dj, di, dj);
-    }
+// Statistic of the counted table in the oracle's order: strata by one thread each, then
+// added in ascending order; every thread returns the sum.  The unit entry point's, and the
+// test kernel's for tables too wide for table_chi2.
+__device__ double table_chi2_ordered(const uint32_t *sm_tab, int dim_s, int di, int dj, double *s_part) {
+    for (int s = threadIdx.x; s < dim_s; s += blockDim.x)
+        s_part[s] = stratum_chi2(sm_tab + (size_t)s * di * dj, di, dj);
     __syncthreads();
     double chi = 0.0;
-    if (threadIdx.x == 0)
-        for (int s = 0; s < dim_s; ++s) chi = __dadd_rn(chi, s_part[s]);
+    for (int s = 0; s < dim_s; ++s) chi = __dadd_rn(chi, s_part[s]);
+    __syncthreads();
+    return chi;
+}
+
+// Statistic of the counted table, all threads of the block; every thread returns the sum.
+// With di, dj <= 32 a thread takes one cell at a time, its marginals summed from the table
+// (integers) and the stratum totals from s_part: q = N N_s - N_a N_b is an exact integer and
+// the cell adds q^2 / (N_a N_b N_s).  A cell costs one FP64 division (GB300's FP64 pipe is
+// 1/64 of its FP32 pipe) and all lanes stay busy; a warp per stratum with its terms added in
+// order took two divisions and a serial chain of additions.  Before that, a lower bound of
+// the sum in FP32 ends tests whose p-value is certainly zero (pvalue_zero; `zero_ok`: a zero
+// p-value changes nothing): *zero is set and 0 returned.
+__device__ double table_chi2(const uint32_t *sm_tab, int dim_s, int di, int dj, double *s_part, bool zero_ok,
+                             bool *zero) {
+    __shared__ double s_red[32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+    *zero = false;
+    if (di > 32 || dj > 32) return table_chi2_ordered(sm_tab, dim_s, di, dj, s_part);
+    double chi = 0.0;
+    uint32_t *s_mt = reinterpret_cast<uint32_t *>(s_part);
+    const int per = di * dj, cells = dim_s * per;
+    for (int s = warp; s < dim_s; s += nwarps) {
+        uint32_t m = 0;
+        for (int k = lane; k < per; k += 32) m += sm_tab[s * per + k];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) m += __shfl_xor_sync(GCSL_FULL_MASK, m, o);
+        if (lane == 0) s_mt[s] = m;
+    }
+    __syncthreads();
+    auto marginals = [&](int k, int &s, uint32_t &ma, uint32_t &mb) {
+        s = k / per;
+        const int r = k - s * per, a = r / dj, b = r - a * dj;
+        const uint32_t *t = sm_tab + s * per;
+        ma = mb = 0;
+        for (int y = 0; y < dj; ++y) ma += t[a * dj + y];
+        for (int x = 0; x < di; ++x) mb += t[x * dj + b];
+    };
+    const int df = (di - 1) * (dj - 1) * dim_s;
+    if (zero_ok && df > 0) {
+        float f = 0.f;
+        for (int k = tid; k < cells; k += blockDim.x) {
+            int s;
+            uint32_t ma, mb;
+            marginals(k, s, ma, mb);
+            if (ma == 0 || mb == 0) continue;
+            const float e = __fdividef((float)ma * (float)mb, (float)s_mt[s]), o = (float)sm_tab[k];
+            f += chi2_floor_term(o, e);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) f += __shfl_xor_sync(GCSL_FULL_MASK, f, o);
+        if (lane == 0) s_red[warp] = (double)f;
+        __syncthreads();
+        float sum = 0.f;
+        for (int w = 0; w < nwarps; ++w) sum += (float)s_red[w];
+        __syncthreads();
+        if (pvalue_zero(0.999f * sum, df)) {
+            *zero = true;
+            return 0.0;
+        }
+    }
+    for (int k = tid; k < cells; k += blockDim.x) {
+        int s;
+        uint32_t ma, mb;
+        marginals(k, s, ma, mb);
+        if (ma == 0 || mb == 0) continue;
+        const long long e = (long long)ma * mb, q = (long long)sm_tab[k] * s_mt[s] - e;
+        chi += (double)q * (double)q / ((double)e * (double)s_mt[s]);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) chi += __shfl_xor_sync(GCSL_FULL_MASK, chi, o);
+    if (lane == 0) s_red[warp] = chi;
+    __syncthreads();
+    chi = 0.0;
+    for (int w = 0; w < nwarps; ++w) chi += s_red[w];
+    __syncthreads();
     return chi;
 }
 
@@ -377,12 +284,18 @@ __device__ __forceinline__ bool table_geometry(const uint8_t *dims, const int *S
     return true;
 }
 
-__global__ void __launch_bounds__(256) disc_test_kernel(DiscLevelArgs A) {
+// Threads of the test kernel: 256 at level 0 (many small tests), 512 above, where the tests
+// are few and large and the block is the parallelism of a test.
+constexpr int DISC_THREADS = 512;
+
+__global__ void __launch_bounds__(DISC_THREADS) disc_test_kernel(DiscLevelArgs A) {
     extern __shared__ uint32_t sm_tab[];
-    __shared__ int s_S[GCSL_MAX_LEVELS + 2];
-    __shared__ int s_mult[GCSL_MAX_LEVELS + 2];
-    __shared__ int s_hdr[7];  // vi, vj, di, dj, dim_s, copies, ok
-    __shared__ long long s_rank;
+    struct Header {
+        int S[GCSL_MAX_LEVELS + 2], mult[GCSL_MAX_LEVELS + 2];
+        int vi, vj, di, dj, dim_s, copies, ok;
+        long long rank;
+    };
+    __shared__ Header s_hdr[2];
     __shared__ int s_bad;
     // per-stratum statistics follow the counters (8-byte aligned)
     double *s_part = reinterpret_cast<double *>(sm_tab + ((A.table_cap + 1) & ~1));
@@ -390,9 +303,9 @@ __global__ void __launch_bounds__(256) disc_test_kernel(DiscLevelArgs A) {
     DevState *st = A.st;
     if (threadIdx.x == 0) {
         s_bad = 0;
-        // codes checked in range for this solve: disc_validate_kernel ran before level 0
-        // and leaves the status 0 only then (any other error also selects the checked
-        // path); read once per CTA, seen by all threads after the first barrier below
+        // codes checked in range for this solve: disc_validate_kernel (or the plane writer) ran
+        // before level 0 and leaves the status 0 only then (any other error also selects the
+        // checked path); read once per CTA, seen by all threads after the first barrier below
         s_trusted = *(volatile const int32_t *)&st->status == 0;
     }
     const int L = A.level;
@@ -408,52 +321,63 @@ __global__ void __launch_bounds__(256) disc_test_kernel(DiscLevelArgs A) {
     const long long total = (L == 0) ? (long long)A.p * (A.p - 1) / 2 : A.prefix[A.p];
     const int tid = threadIdx.x;
 
-    for (long long t0 = blockIdx.x; t0 < total; t0 += gridDim.x) {
+    // test t0's variables and table geometry (one thread)
+    auto prepare = [&](long long t0, Header &H) {
         const long long t = work_order(t0, total, A.order);
-        if (tid == 0) {
-            int vi, vj;
-            long long rank = 0;
-            if (L == 0) {
-                tri_pair(t, vi, vj);
-            } else {
-                vi = upper_row(A.prefix, A.p, t);
-                const long long off = t - A.prefix[vi];
-                const int deg = A.adj[(size_t)vi * A.p];
-                const long long R = binom_rt(deg - 1, L);
-                const int m = (int)(off / R);
-                rank = off - (long long)m * R;
-                vj = A.adj[(size_t)vi * A.p + 1 + m];
-                unrank_positions_rt(L, deg - 1, rank, s_S);
-                const int *nbrs = A.adj + (size_t)vi * A.p + 1;
-                for (int c = 0; c < L; ++c) s_S[c] = resolve_position(nbrs, vj, s_S[c]);
-            }
-            int dim_s = 0, di = 0, dj = 0, copies = 1;
-            const bool ok =
-                table_geometry(A.dims, s_S, s_mult, L, vi, vj, A.table_cap, A.part_cap, dim_s, di, dj, copies);
-            s_hdr[0] = vi;
-            s_hdr[1] = vj;
-            s_hdr[2] = di;
-            s_hdr[3] = dj;
-            s_hdr[4] = dim_s;
-            s_hdr[5] = copies;
-            s_hdr[6] = ok;
-            s_rank = rank;
-            if (!ok) set_status(st, GCSL_ERR_UNSUPPORTED);
+        int vi, vj;
+        long long rank = 0;
+        if (L == 0) {
+            tri_pair(t, vi, vj);
+        } else {
+            vi = upper_row(A.prefix, A.p, t);
+            const long long off = t - A.prefix[vi];
+            const int deg = A.adj[(size_t)vi * A.p];
+            const long long R = binom_rt(deg - 1, L);
+            const int m = (int)(off / R);
+            rank = off - (long long)m * R;
+            vj = A.adj[(size_t)vi * A.p + 1 + m];
+            unrank_positions_rt(L, deg - 1, rank, H.S);
+            const int *nbrs = A.adj + (size_t)vi * A.p + 1;
+            for (int c = 0; c < L; ++c) H.S[c] = resolve_position(nbrs, vj, H.S[c]);
         }
+        int dim_s = 0, di = 0, dj = 0, copies = 1;
+        const bool ok =
+            table_geometry(A.dims, H.S, H.mult, L, vi, vj, A.table_cap, A.part_cap, dim_s, di, dj, copies);
+        H.vi = vi;
+        H.vj = vj;
+        H.di = di;
+        H.dj = dj;
+        H.dim_s = dim_s;
+        H.copies = copies;
+        H.ok = ok;
+        H.rank = rank;
+        if (!ok) set_status(st, GCSL_ERR_UNSUPPORTED);
+    };
+
+    // the next test's header is prepared by the last warp while the others start on this one's
+    // statistic
+    if (tid == 0 && blockIdx.x < total) prepare(blockIdx.x, s_hdr[0]);
+    int cur = 0;
+    for (long long t0 = blockIdx.x; t0 < total; t0 += gridDim.x, cur ^= 1) {
         __syncthreads();
-        if (!s_hdr[6]) {
-            __syncthreads();
+        const Header &H = s_hdr[cur];
+        const bool more = t0 + gridDim.x < total;
+        const int ahead = blockDim.x - 32;  // the thread that prepares
+        if (!H.ok) {
+            if (tid == ahead && more) prepare(t0 + gridDim.x, s_hdr[cur ^ 1]);
             continue;
         }
-        const int vi = s_hdr[0], vj = s_hdr[1], di = s_hdr[2], dj = s_hdr[3], dim_s = s_hdr[4];
-        count_table(A.data, A.ld, A.n, vi, vj, s_S, s_mult, L, di, dj, dim_s * di * dj, s_hdr[5], sm_tab,
-                    &s_bad, s_trusted != 0);
-        const double chi = table_chi2(sm_tab, dim_s, di, dj, s_part);
+        const int vi = H.vi, vj = H.vj, di = H.di, dj = H.dj, dim_s = H.dim_s;
+        count_table(A.data, A.ld, A.n, vi, vj, H.S, H.mult, L, di, dj, dim_s * di * dj, H.copies, sm_tab, &s_bad,
+                    s_trusted != 0);
+        if (tid == ahead && more) prepare(t0 + gridDim.x, s_hdr[cur ^ 1]);
+        bool zero;
+        const double chi = table_chi2(sm_tab, dim_s, di, dj, s_part, A.alpha > 0.0, &zero);
         if (tid == 0 && s_bad) set_status(st, GCSL_ERR_INVALID_ARG);
-        double pv = 1.0;
-        if (tid < 32) {  // warp 0: the p-value's series split over the lanes
+        double pv = 0.0;
+        if (!zero && tid < 32) {  // warp 0: the p-value's series split over the lanes
             const long long df = (long long)(di - 1) * (long long)(dj - 1) * (long long)dim_s;
-            pv = pchisq_warp(__shfl_sync(GCSL_FULL_MASK, chi, 0), df);
+            pv = pchisq_tab_warp(chi, df, A.lg);
         }
         if (tid == 0) {
             const int lo = vi < vj ? vi : vj, hi = vi < vj ? vj : vi;
@@ -463,15 +387,14 @@ __global__ void __launch_bounds__(256) disc_test_kernel(DiscLevelArgs A) {
                 const uint16_t keep = (pv >= A.alpha) ? 0 : 1;
                 A.G[(size_t)vi * A.p + vj] = keep;
                 A.G[(size_t)vj * A.p + vi] = keep;
-            } else {
+            } else if (!zero) {
                 atomic_max_nonneg(&A.pmax[ix], pv);
                 if (pv >= A.alpha) {
-                    const unsigned long long key = ((unsigned long long)s_rank << 1) | (vi < vj ? 0ull : 1ull);
+                    const unsigned long long key = ((unsigned long long)H.rank << 1) | (vi < vj ? 0ull : 1ull);
                     atomicMin(&A.win[ix], key);
                 }
             }
         }
-        __syncthreads();
     }
     if (blockIdx.x == 0 && tid == 0) st->tests[L] = (unsigned long long)total;
 }
@@ -511,7 +434,7 @@ __global__ void __launch_bounds__(256) disc_table_kernel(const uint8_t *data, lo
     if (threadIdx.x == 0) s_bad = 0;
     count_table(data, ld, n, vi, vj, s_S, s_mult, L, di, dj, T, s_hdr[3], sm_tab, &s_bad, false);
     for (int k = threadIdx.x; k < T; k += blockDim.x) counts[k] = sm_tab[k];
-    const double chi = table_chi2(sm_tab, dim_s, di, dj, s_part);
+    const double chi = table_chi2_ordered(sm_tab, dim_s, di, dj, s_part);
     if (threadIdx.x == 0) {
         if (s_bad) {
             out2[0] = out2[1] = -1.0;
@@ -522,7 +445,6 @@ __global__ void __launch_bounds__(256) disc_table_kernel(const uint8_t *data, lo
     }
 }
 
-// Per-row weights deg_r * C(deg_r - 1, L) of the level's flattened test list.
 // Codes in range: every code of columns 0..p-1 (samples 0..n-1) below its cardinality.
 // Sets GCSL_ERR_INVALID_ARG otherwise, which makes the test kernels check every sample.
 // A byte x of a word is >= d (1 <= d <= 128) iff the high bit of (x + 128 - d) | x is
@@ -530,7 +452,8 @@ __global__ void __launch_bounds__(256) disc_table_kernel(const uint8_t *data, lo
 // may carry) has its own high bit set, so the word test is exact.
 __global__ void __launch_bounds__(256) disc_validate_kernel(const uint8_t *__restrict__ data, long long ld,
                                                             long long n, int p, const uint8_t *__restrict__ dims,
-                                                            DevState *st) {
+                                                            double *__restrict__ lg, DevState *st) {
+    if (blockIdx.x < LG_BLOCKS) lgam_build(lg, (int)blockIdx.x);
     const long long nvec = (n + 15) >> 4;
     const long long total = nvec * p;
     bool bad = false;
@@ -555,15 +478,48 @@ __global__ void __launch_bounds__(256) disc_validate_kernel(const uint8_t *__res
     if (__any_sync(GCSL_FULL_MASK, bad) && (threadIdx.x & 31) == 0) set_status(st, GCSL_ERR_INVALID_ARG);
 }
 
-__global__ void disc_weights_kernel(const int *__restrict__ adj, int p, int L, long long *__restrict__ w,
-                                    DevState *st) {
+// One block plans a level: per-row test counts deg C(deg - 1, L) and their exclusive prefix,
+// the edge and test totals, and with group > 0 the bit-plane path's tasks (pairs of a row's
+// neighbour groups of `group` variables): `rows` lists the rows by falling work, about d deg^2,
+// so that the uneven tasks are started largest first, and `tasks` is the prefix of their task
+// counts in that order.
+__global__ void __launch_bounds__(1024) disc_plan_kernel(const int *__restrict__ adj, int p, int L, int group,
+                                                         const uint8_t *__restrict__ dims, long long *__restrict__ w,
+                                                         long long *__restrict__ prefix, long long *__restrict__ tasks,
+                                                         int *__restrict__ rows, DevState *st) {
+    extern __shared__ long long s_key[];
     if (st->done) return;
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= p) return;
-    const int deg = adj[(size_t)r * p];
-    const long long R = (deg - 1 >= L) ? binom_rt(deg - 1, L) : 0;
-    if (R >= GCSL_RANK_LIMIT) set_status(st, GCSL_ERR_UNSUPPORTED);
-    w[r] = (long long)deg * R;
+    unsigned long long edges = 0;
+    for (int r = threadIdx.x; r < p; r += blockDim.x) {
+        const int deg = adj[(size_t)r * p];
+        const long long R = (deg - 1 >= L) ? binom_rt(deg - 1, L) : 0;
+        if (R >= GCSL_RANK_LIMIT) set_status(st, GCSL_ERR_UNSUPPORTED);
+        w[r] = (long long)deg * R;
+        edges += (unsigned long long)deg;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) edges += __shfl_xor_sync(GCSL_FULL_MASK, edges, o);
+    if ((threadIdx.x & 31) == 0 && edges) atomicAdd(&st->edges[L], edges);  // directed count; halved on the host
+    __syncthreads();
+    block_scan_rows(w, p, prefix);
+    __syncthreads();
+    if (threadIdx.x == 0) st->tests_full[L] = (unsigned long long)prefix[p];
+    if (group <= 0) return;
+    for (int r = threadIdx.x; r < p; r += blockDim.x) {
+        const long long deg = adj[(size_t)r * p];
+        s_key[r] = w[r] > 0 ? deg * deg * dims[r] : 0;
+    }
+    __syncthreads();
+    for (int r = threadIdx.x; r < p; r += blockDim.x) {
+        const long long key = s_key[r];
+        int rank = 0;
+        for (int q = 0; q < p; ++q) rank += s_key[q] > key || (s_key[q] == key && q < r);
+        const long long ng = key > 0 ? (adj[(size_t)r * p] + group - 1) / group : 0;
+        rows[rank] = r;
+        w[rank] = ng * (ng + 1) / 2;
+    }
+    __syncthreads();
+    block_scan_rows(w, p, tasks);
 }
 
 // Write-back of a level: canonical remover -> skeleton, sepsets, records.
@@ -608,17 +564,6 @@ __global__ void disc_finalize_kernel(const int *__restrict__ adj, int p, int L, 
         ++removed;
     }
     if (removed) atomicAdd(&st->removed[L], removed);
-}
-
-// Edges alive at level start and the level's full test space (for the stats).
-__global__ void disc_level_stats_kernel(const long long *__restrict__ prefix, const int *__restrict__ adj, int p,
-                                        int L, DevState *st) {
-    if (st->done) return;
-    if (threadIdx.x == 0 && blockIdx.x == 0) st->tests_full[L] = (unsigned long long)prefix[p];
-    unsigned long long e = 0;
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < p; r += gridDim.x * blockDim.x)
-        e += (unsigned long long)adj[(size_t)r * p];
-    if (e) atomicAdd(&st->edges[L], e);  // directed count; halved on the host
 }
 
 __global__ void pmax_finish_kernel(double *pmax, int p) {
@@ -673,25 +618,30 @@ cudaError_t launch_disc_tests(const DiscLevelArgs &A, int num_sms, cudaStream_t 
     const cudaError_t ea = raise_dyn_smem_limit(disc_test_kernel, limit_set);
     if (ea != cudaSuccess) return note_error("disc_test_kernel shared memory", ea);
     int per_sm = 1;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, disc_test_kernel, 256, smem) != cudaSuccess ||
+    const int threads = A.level == 0 ? DISC_THREADS / 2 : DISC_THREADS;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, disc_test_kernel, threads, smem) != cudaSuccess ||
         per_sm < 1)
         per_sm = 1;
     const int cap = blocks_per_sm_cap();  // room left on every SM for concurrent solves
     if (cap > 0 && per_sm > cap) per_sm = cap;
-    disc_test_kernel<<<num_sms * per_sm, 256, smem, s>>>(A);
+    disc_test_kernel<<<num_sms * per_sm, threads, smem, s>>>(A);
     note_launch(1);
     return note_error("disc_test_kernel launch", cudaGetLastError());
 }
 
+// Also builds the ln Gamma tables (at least LG_BLOCKS blocks: num_sms >= 1).
 cudaError_t launch_disc_validate(const uint8_t *data, long long ld, long long n, int p, const uint8_t *dims,
-                                 DevState *st, int num_sms, cudaStream_t s) {
-    disc_validate_kernel<<<num_sms * 4, 256, 0, s>>>(data, ld, n, p, dims, st);
+                                 double *lg, DevState *st, int num_sms, cudaStream_t s) {
+    disc_validate_kernel<<<std::max(num_sms * 4, LG_BLOCKS), 256, 0, s>>>(data, ld, n, p, dims, lg, st);
     note_launch(1);
     return note_error("disc_validate_kernel launch", cudaGetLastError());
 }
 
-cudaError_t launch_disc_weights(const int *adj, int p, int L, long long *w, DevState *st, cudaStream_t s) {
-    disc_weights_kernel<<<(p + 255) / 256, 256, 0, s>>>(adj, p, L, w, st);
+// group: neighbours per group of the bit-plane path's level 1 (0: no tasks).
+cudaError_t launch_disc_plan(const int *adj, int p, int L, int group, const uint8_t *dims, long long *w,
+                             long long *prefix, long long *tasks, int *rows, DevState *st, cudaStream_t s) {
+    const size_t smem = group > 0 ? (size_t)p * sizeof(long long) : 0;  // p <= 4096 with groups
+    disc_plan_kernel<<<1, 1024, smem, s>>>(adj, p, L, group, dims, w, prefix, tasks, rows, st);
     note_launch(1);
     return cudaGetLastError();
 }
@@ -700,13 +650,6 @@ cudaError_t launch_disc_finalize(const int *adj, int p, int L, uint16_t *G, unsi
                                  int max_level, int *rec, long long rec_cap, DevState *st, int num_sms,
                                  cudaStream_t s) {
     disc_finalize_kernel<<<num_sms * 2, 256, 0, s>>>(adj, p, L, G, win, sep, max_level, rec, rec_cap, st);
-    note_launch(1);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_disc_level_stats(const long long *prefix, const int *adj, int p, int L, DevState *st,
-                                    cudaStream_t s) {
-    disc_level_stats_kernel<<<(p + 255) / 256, 256, 0, s>>>(prefix, adj, p, L, st);
     note_launch(1);
     return cudaGetLastError();
 }

@@ -356,12 +356,6 @@ cudaError_t launch_scan_int(const int *cnt, int p, long long *prefix, DevState *
     return cudaGetLastError();
 }
 
-cudaError_t launch_scan_ll(const long long *cnt, int p, long long *prefix, DevState *st, cudaStream_t s) {
-    row_scan_kernel<long long><<<1, 1024, 0, s>>>(cnt, p, prefix, st);
-    note_launch(1);
-    return cudaGetLastError();
-}
-
 // The level's context (thresholds, FP32 bounds of the knife edge, queue) for launches.
 LevelCtx level_ctx(int L, const double *C, int p, const int *adj, const int2 *elist, double tau, bool tau_valid,
                    uint16_t *G, double *zmin, double *r2min, int *sep_dense, int max_level, int *rec_pool,
