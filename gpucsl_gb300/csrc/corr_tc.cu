@@ -662,12 +662,15 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
         if (ok) {
             const int row = qd * 32 + lane;
             const size_t base = ((size_t)split * D.p_pad + (size_t)(I * OZ_TM + row)) * D.p_pad + J * OZ_TN + cq * 16;
-            long long *__restrict__ part_hi = s_job.phi;
-            long long *__restrict__ part_lo = s_job.plo;
+            // two words a store (base is a multiple of 16); rows and columns past p are never read
+            longlong2 *__restrict__ part_hi = reinterpret_cast<longlong2 *>(s_job.phi + base);
+            longlong2 *__restrict__ part_lo = reinterpret_cast<longlong2 *>(s_job.plo + base);
+            if (I * OZ_TM + row < D.p && J * OZ_TN + cq * 16 < D.p) {
 #pragma unroll
-            for (int e = 0; e < 16; ++e) {
-                part_hi[base + e] = acc_hi[e];
-                part_lo[base + e] = acc_lo[e];
+                for (int e = 0; e < 8; ++e) {
+                    part_hi[e] = make_longlong2(acc_hi[2 * e], acc_hi[2 * e + 1]);
+                    part_lo[e] = make_longlong2(acc_lo[2 * e], acc_lo[2 * e + 1]);
+                }
             }
         }
     }
@@ -727,17 +730,33 @@ __device__ __forceinline__ double scale_pow2(double x, int e) {
     return __longlong_as_double(b + ((long long)e << 52));
 }
 
-// Covariance of (i, j) from the exact split sums: (2^28 H + L) 2^(E_i + E_j - 56) / (n - 1).
-__device__ __forceinline__ double oz_cov(const long long *__restrict__ part_hi, const long long *__restrict__ part_lo,
-                                         const OzDims &D, const int *__restrict__ expo, double scale, int i, int j) {
-    long long H = 0, Lo = 0;
-    for (int s = 0; s < D.splits; ++s) {
-        const size_t ix = ((size_t)s * D.p_pad + i) * D.p_pad + j;
-        H += part_hi[ix];
-        Lo += part_lo[ix];
+// Exact split sums (H, L) of entry ix of a split (p_pad^2 words apart), four splits' loads in
+// flight at a time.
+__device__ __forceinline__ void split_sums(const long long *__restrict__ part_hi, const long long *__restrict__ part_lo,
+                                           const OzDims &D, size_t ix, long long &H, long long &Lo) {
+    const size_t step = (size_t)D.p_pad * D.p_pad;
+    H = Lo = 0;
+    int s = 0;
+    for (; s + 4 <= D.splits; s += 4) {
+        long long h[4], l[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            h[e] = part_hi[ix + (s + e) * step];
+            l[e] = part_lo[ix + (s + e) * step];
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) H += h[e], Lo += l[e];
     }
+    for (; s < D.splits; ++s) {
+        H += part_hi[ix + s * step];
+        Lo += part_lo[ix + s * step];
+    }
+}
+
+// Covariance of (i, j) from the exact sums: (2^28 H + L) 2^(E_i + E_j - 56) / (n - 1).
+__device__ __forceinline__ double oz_cov(long long H, long long Lo, int ei, int ej, double scale) {
     const double val = exact_sum_to_f64(H, Lo);  // exact terms, one rounding
-    return scale_pow2(val, expo[i] + expo[j] - 56) * scale;
+    return scale_pow2(val, ei + ej - 56) * scale;
 }
 
 // Bound of |C' - C| for the five-digit product C' against the seven-digit C, from the
@@ -754,13 +773,7 @@ __device__ __forceinline__ double oz_cov(const long long *__restrict__ part_hi, 
 // normalisation by the (equally perturbed) variances at most doubles it to first
 // order; the factor 2.5 covers that, the higher-order terms and the roundings.
 template <class Src>
-__device__ __forceinline__ double split_eps(const OzJob &J, int i) {
-    long long H = 0, Lo = 0;
-    for (int s = 0; s < J.D.splits; ++s) {
-        const size_t ix = ((size_t)s * J.D.p_pad + i) * J.D.p_pad + i;
-        H += J.phi[ix];
-        Lo += J.plo[ix];
-    }
+__device__ __forceinline__ double split_eps(const OzJob &J, long long H, long long Lo) {
     const double S = scale_pow2(exact_sum_to_f64(H, Lo), -56);  // sum_t y_ti^2
     if (!(S > 0.0)) return __longlong_as_double(0x7ff0000000000000ll);
     const double w = (double)J.n / S;
@@ -777,11 +790,13 @@ __global__ void ozaki_diag_kernel(Src src) {
     const int i = (int)lb * blockDim.x + threadIdx.x;
     const double scale = 1.0 / (double)(J.n - 1);
     if (i < J.p) {
-        J.inv_sd[i] = 1.0 / sqrt(oz_cov(J.phi, J.plo, J.D, J.expo, scale, i, i));
+        long long H, Lo;
+        split_sums(J.phi, J.plo, J.D, (size_t)i * J.D.p_pad + i, H, Lo);
+        J.inv_sd[i] = 1.0 / sqrt(oz_cov(H, Lo, J.expo[i], J.expo[i], scale));
         double *slot = src.err_slot(J.index);
         if (slot != nullptr)  // non-negative doubles order like their bit patterns
             atomicMax(reinterpret_cast<unsigned long long *>(slot),
-                      (unsigned long long)__double_as_longlong(split_eps<Src>(J, i)));
+                      (unsigned long long)__double_as_longlong(split_eps<Src>(J, H, Lo)));
     }
 }
 
@@ -789,8 +804,14 @@ __global__ void ozaki_diag_kernel(Src src) {
 // reciprocals of the standard deviations), for one 32 x 32 tile of the upper triangle
 // per block; the mirrored tile is written through shared memory so both triangles are
 // stored row-contiguously, and the FP32 copy the same way when the job has one.
+//
+// Bound by the latency of the partial sums' loads: a thread issues those of its four entries
+// (of two splits at a time) before it uses one; three blocks per SM keep 16 loads a thread
+// in registers.  A loop that used each load at once cost 110 us at p = 20 (one block, 63
+// splits; now 8.5 us with 8), 61 us at p = 211 (25 splits; now 19 us) and 245 us at p = 5000
+// (one split; now 191 us, 400 MB moved).
 template <class Src>
-__global__ void ozaki_finish_kernel(Src src) {
+__global__ void __launch_bounds__(256, 3) ozaki_finish_kernel(Src src) {
     __shared__ double tv[32][33];
     pdl_wait();
     pdl_trigger();
@@ -808,11 +829,50 @@ __global__ void ozaki_finish_kernel(Src src) {
     const double scale = 1.0 / (double)(J.n - 1);
     const bool failed = *J.err != 0;  // a tensor-core wait timed out: poison the output
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    for (int r = ty; r < 32; r += 8) {
-        const int i = bi * 32 + r, j = bj * 32 + tx;
+    const int j = bj * 32 + tx;
+    const size_t pitch = (size_t)J.D.p_pad, step = pitch * pitch;
+    const int ej = j < p ? J.expo[j] : 0;
+    const double sj = j < p ? J.inv_sd[j] : 0.0;
+    long long H[4], Lo[4];
+    int ei[4];
+    double si[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int i = bi * 32 + ty + 8 * q;
+        H[q] = Lo[q] = 0;
+        ei[q] = i < p ? J.expo[i] : 0;
+        si[q] = i < p ? J.inv_sd[i] : 0.0;
+    }
+    // Every lane loads, rows and columns past p those of p - 1 (a branch around a load would
+    // serialise the loads); entries below the diagonal of a diagonal tile exist as well.
+    size_t at[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) at[q] = (size_t)min(bi * 32 + ty + 8 * q, p - 1) * pitch + min(j, p - 1);
+    const long long *__restrict__ hi = J.phi, *__restrict__ lo = J.plo;
+    const int splits = J.D.splits;
+    int s = 0;
+    for (; s + 2 <= splits; s += 2) {
+        long long h[8], l[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            h[q] = hi[at[q & 3] + (q >> 2) * step];
+            l[q] = lo[at[q & 3] + (q >> 2) * step];
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) H[q & 3] += h[q], Lo[q & 3] += l[q];
+        hi += 2 * step;
+        lo += 2 * step;
+    }
+    if (s < splits) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) H[q] += hi[at[q]], Lo[q] += lo[at[q]];
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int r = ty + 8 * q, i = bi * 32 + r;
         double v = 0.0;
         if (i < p && j < p && (bi != bj || i <= j)) {
-            v = oz_cov(J.phi, J.plo, J.D, J.expo, scale, i, j) * J.inv_sd[i] * J.inv_sd[j];
+            v = oz_cov(H[q], Lo[q], ei[q], ej, scale) * si[q] * sj;
             // clip to [-1, 1] on the bits, as fmin(fmax(v, -1), 1) (NaN gives -1)
             const unsigned long long vb = (unsigned long long)__double_as_longlong(v);
             const unsigned long long mag = vb & 0x7fffffffffffffffull;
@@ -836,6 +896,11 @@ __global__ void ozaki_finish_kernel(Src src) {
 
 namespace host {
 
+// A split of a small job takes at least this many K steps: a step costs about half a
+// microsecond, and every further split adds 16 bytes per entry to write and to sum again
+// (p = 20, n = 1000: 63 splits of one step against 8 of eight).
+constexpr int OZ_MIN_STEPS = 8;
+
 // splits: K splits of the tile grid; 0 chooses one wave over num_sms SMs
 static OzDims oz_dims(long long n, int p, int num_sms, int splits_req = 0) {
     OzDims D;
@@ -849,6 +914,8 @@ static OzDims oz_dims(long long n, int p, int num_sms, int splits_req = 0) {
     const long long steps = D.n_pad / 16;
     int splits = splits_req > 0 ? splits_req : num_sms / tiles;  // one wave: tiles x splits <= SMs
     if (splits < 1) splits = 1;
+    if (splits_req <= 0 && splits > (steps + OZ_MIN_STEPS - 1) / OZ_MIN_STEPS)
+        splits = (int)((steps + OZ_MIN_STEPS - 1) / OZ_MIN_STEPS);
     if (splits > steps) splits = (int)steps;
     D.slabs_per_split = (int)((steps + splits - 1) / splits);
     D.splits = (int)((steps + D.slabs_per_split - 1) / D.slabs_per_split);
