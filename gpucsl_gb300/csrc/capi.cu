@@ -20,7 +20,8 @@ namespace gcsl {
 namespace host {
 cudaError_t launch_level0(const double *C, int p, double tau0, uint16_t *G, double *zmin, double *r2min, int *kept,
                           DevState *st, float *C32, cudaStream_t s);
-cudaError_t launch_sf_table(double *out, cudaStream_t s);
+cudaError_t launch_sf_table(double *out, double *rt, int p, long long n_obs, double tau, cudaStream_t s);
+size_t pmax_table_doubles();
 cudaError_t launch_compact(const uint16_t *G, int p, int *adj, int *up, DevState *st, int level, int2 *elist,
                            cudaStream_t s);
 cudaError_t launch_scan_int(const int *cnt, int p, long long *prefix, DevState *st, cudaStream_t s);
@@ -41,11 +42,10 @@ cudaError_t orient_edges(const uint16_t *S, int p, const int *sep, int L, uint8_
 cudaError_t launch_cand(int L, const double *C, int p, double tau, double *zmin, double *r2min, const int *qbuf,
                         long long qcap, DevState *st, const long long *chunk_first, int num_sms, cudaStream_t s);
 cudaError_t launch_pmax(const int *kept, const DevState *st, const double *zmin, const double *r2min, int p,
-                        long long n_obs, const double *sftab, double *pmax, int num_sms,
+                        long long n_obs, const double *sftab, const double *rt, double tau, double *pmax, int num_sms,
                         cudaStream_t s);
 cudaError_t launch_pmax_level0(const double *C, const double *zmin, int p, long long n_obs, const double *sftab,
-                               double *pmax,
-                               int num_sms, cudaStream_t s);
+                               const double *rt, double tau, double *pmax, int num_sms, cudaStream_t s);
 size_t corr_workspace_bytes(long long n, int p);
 cudaError_t corr_f64(const void *X, int dtype, long long n, int p, long long ldx, double *C, void *ws,
                      size_t ws_bytes, int num_sms, cudaStream_t s);
@@ -432,6 +432,7 @@ struct GaussWs {
     int2 *elist;      // the level's edges (lo, hi)
     float *c32;       // FP32 copy of C for the FP32-first tests
     double *sftab;    // erfc Taylor table of the pmax kernels
+    double *rt;       // their table of pmax by |rho|
     int *cand;        // FP64 z* candidate queue
     long long cand_cap;
     ChunkBufs ck;     // chunked edges of the current level (chunk_first: one region per level)
@@ -493,6 +494,7 @@ GaussWs carve_gauss(void *ws, size_t cap, int p) {
     w.elist = c.take<int2>((size_t)p * (p - 1) / 2 + 1);
     w.c32 = c.take<float>((size_t)p * p);
     w.sftab = c.take<double>(32 * 13);
+    w.rt = c.take<double>(host::pmax_table_doubles());
     w.cand_cap = cand_queue_ints(p);
     w.cand = c.take<int>((size_t)w.cand_cap);
     w.ck.heavy_cap = chunk_edges_cap(p);
@@ -645,8 +647,12 @@ int gcsl::host::gauss_skeleton_run(const double *C, int p, long long n_obs, cons
         joiner.armed = true;  // from here every return joins the side stream back into s
     }
     cudaStream_t aux = ss ? ss->stream : s;
-    if (host::launch_sf_table(w.sftab, aux) != cudaSuccess ||
-        host::launch_pmax_level0(C, w.zmin, p, n_obs, w.sftab, pmax, sms, aux) != cudaSuccess)
+    // the largest threshold of the levels that run (they rise slowly with the level)
+    double tau_max = 0.0;
+    for (int l = 0; l <= std::min({max_level, n_thresholds - 1, GCSL_GAUSS_REG_LEVELS}); ++l)
+        tau_max = std::max(tau_max, thresholds[l]);
+    if (host::launch_sf_table(w.sftab, w.rt, p, n_obs, tau_max, aux) != cudaSuccess ||
+        host::launch_pmax_level0(C, w.zmin, p, n_obs, w.sftab, w.rt, tau_max, pmax, sms, aux) != cudaSuccess)
         return GCSL_ERR_DEVICE;
     const long long region = cand_region_ints(w.cand_cap);
     auto enqueue_on = [&](int level, cudaStream_t s) -> cudaError_t {
@@ -718,7 +724,7 @@ int gcsl::host::gauss_skeleton_run(const double *C, int p, long long n_obs, cons
     const int rc = run_levels(max_level, w.st, s, words, enqueue_range);
     if (joiner.join() != cudaSuccess) return GCSL_ERR_DEVICE;
     if (rc != GCSL_OK) return rc;
-    if (host::launch_pmax(w.kept, w.st, w.zmin, w.r2min, p, n_obs, w.sftab, pmax, sms, s) != cudaSuccess)
+    if (host::launch_pmax(w.kept, w.st, w.zmin, w.r2min, p, n_obs, w.sftab, w.rt, tau_max, pmax, sms, s) != cudaSuccess)
         return GCSL_ERR_DEVICE;
     const int frc = finish_stats(w.st, stats, s, false, p);
     if (lt) {

@@ -265,50 +265,49 @@ __global__ void __launch_bounds__(128) gauss_level_smem_kernel(const double *__r
 // pmax_ij = 2 * sf(sqrt(n - 3) * z*_ij) for i < j (0 when z* = +inf), -1 elsewhere.
 // 2 sf(x) = erfc(x / sqrt 2), written as scipy's ndtr does it (erf below 1/sqrt 2).
 // Grid: (column blocks of 256, rows); no index division.
-// The erfc Taylor table of the pmax kernels, built once per solve by one warp.
-__global__ void sf_table_kernel(double *__restrict__ out) {
+// The tables of the pmax kernels, built once per solve: block 0 the erfc table, blocks 1 ..
+// (with a table of f) its centres, one per thread.
+__global__ void sf_table_kernel(double *__restrict__ out, RTab R, double *__restrict__ rt) {
+    if (blockIdx.x > 0) {
+        const int m = (blockIdx.x - 1) * blockDim.x + threadIdx.x;
+        if (m < RT_CENTRES) rt_build(R, m, rt + m * RT_TERMS);
+        return;
+    }
     __shared__ double tab[SF_CENTRES][SF_TERMS];
     sf_table_build(tab);
     __syncthreads();
     for (int k = threadIdx.x; k < SF_CENTRES * SF_TERMS; k += blockDim.x) out[k] = (&tab[0][0])[k];
 }
 
-// Pairs kept at level 0 (the list the level-0 kernel appended): z* = min(zmin, Z of the
-// smallest rho^2 any later level stored), pmax = 2 sf(sqrt(n - 3) z*)
-// (helpers.py:62-82 with the FP64 z*).
-__global__ void pmax_kept_kernel(const int *__restrict__ kept, const DevState *__restrict__ st,
-                                 const double *__restrict__ zmin, const double *__restrict__ r2min, double sqrt_nm3,
-                                 const double *__restrict__ sftab, double *__restrict__ pmax) {
-    __shared__ double tab[SF_CENTRES][SF_TERMS];
-    sf_table_load(tab, sftab);
+// Pairs kept at level 0 (the list the level-0 kernel appended).
+__global__ void __launch_bounds__(256) pmax_kept_kernel(const int *__restrict__ kept, const DevState *__restrict__ st,
+                                                        const double *__restrict__ zmin,
+                                                        const double *__restrict__ r2min, double sqrt_nm3,
+                                                        const double *__restrict__ sftab, RTab R,
+                                                        double *__restrict__ pmax) {
+    __shared__ PmaxShared S;
+    const int n = st->n_kept;
+    if ((int)(blockIdx.x * blockDim.x) >= n) return;
+    pmax_tables_load(S, sftab, R);
     __syncthreads();
-    const int count = st->n_kept;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < count; t += gridDim.x * blockDim.x) {
-        const int k = kept[t];
-        double z = zmin[k];
-        const double r2 = r2min[k];
-        if (r2 < 1.0) z = fmin(z, fisher_z(sqrt(r2)));  // Z increasing in rho^2 below 1
-        pmax[k] = two_sf_tab(sqrt_nm3 * z, tab);
-    }
+    pmax_kept_share(S, R, kept, n, zmin, r2min, sqrt_nm3, pmax, (int)blockIdx.x, (int)gridDim.x);
 }
 
 // Every other entry: pairs removed at level 0 (marker zmin = -1) get z* = Z(r) with
 // r = C[i*p + j] (gaussian_ci.cu:36-37), the lower triangle and diagonal -1.  Launched on
 // a second stream right after level 0; the later levels never touch these entries, so it
-// runs concurrently with them.
-__global__ void pmax_level0_kernel(const double *__restrict__ C, const double *__restrict__ zmin, int p,
-                                   double sqrt_nm3, const double *__restrict__ sftab, double *__restrict__ pmax) {
-    __shared__ double tab[SF_CENTRES][SF_TERMS];
-    sf_table_load(tab, sftab);
+// runs concurrently with them.  FP64 pipe: 785 us at p = 5000 with the two-step evaluation.
+__global__ void __launch_bounds__(256) pmax_level0_kernel(const double *__restrict__ C, const double *__restrict__ zmin,
+                                                          int p, double sqrt_nm3, const double *__restrict__ sftab,
+                                                          RTab R, double *__restrict__ pmax) {
+    __shared__ PmaxShared S;
+    pmax_tables_load(S, sftab, R);
     __syncthreads();
     const unsigned total = (unsigned)p * (unsigned)p;  // p <= 46340: fits in 31 bits
     for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k < total; k += gridDim.x * blockDim.x) {
         const int i = (int)(k / (unsigned)p), j = (int)(k - (unsigned)i * (unsigned)p);
-        if (i >= j) {
-            pmax[k] = -1.0;
-        } else if (zmin[k] < 0.0) {
-            pmax[k] = two_sf_tab(sqrt_nm3 * fisher_z(C[k]), tab);
-        }
+        if (i >= j) pmax[k] = -1.0;
+        else if (zmin[k] < 0.0) pmax[k] = pmax_removed(S, R, sqrt_nm3, C[k]);
     }
 }
 
@@ -494,28 +493,36 @@ cudaError_t launch_unrank(int K, int L, long long count, int *out, cudaStream_t 
     return cudaGetLastError();
 }
 
-cudaError_t launch_sf_table(double *out, cudaStream_t s) {
-    sf_table_kernel<<<1, 32, 0, s>>>(out);
+// rt: RT_CENTRES x RT_TERMS doubles for the table of f (gauss_dev.cuh); tau: the largest
+// threshold of the solve.  The same arguments give launch_pmax* their table.
+cudaError_t launch_sf_table(double *out, double *rt, int p, long long n_obs, double tau, cudaStream_t s) {
+    const RTab R = rt_params(n_obs, tau, (long long)p * (p - 1) / 2, rt);
+    sf_table_kernel<<<R.a != nullptr ? 1 + RT_CENTRES / 32 : 1, 32, 0, s>>>(out, R, rt);
     note_launch(1);
     return cudaGetLastError();
 }
 
+size_t pmax_table_doubles() { return (size_t)RT_CENTRES * RT_TERMS; }
+
 cudaError_t launch_pmax_level0(const double *C, const double *zmin, int p, long long n_obs, const double *sftab,
-                               double *pmax, int num_sms, cudaStream_t s) {
+                               const double *rt, double tau, double *pmax, int num_sms, cudaStream_t s) {
     const long long total = (long long)p * p;
     const long long want = (total + 255) / 256;
     const int blocks = (int)(want < (long long)num_sms * 4 ? want : (long long)num_sms * 4);
-    pmax_level0_kernel<<<blocks > 0 ? blocks : 1, 256, 0, s>>>(C, zmin, p, sqrt((double)(n_obs - 3)), sftab, pmax);
+    const RTab R = rt_params(n_obs, tau, (long long)p * (p - 1) / 2, rt);
+    pmax_level0_kernel<<<blocks > 0 ? blocks : 1, 256, 0, s>>>(C, zmin, p, sqrt((double)(n_obs - 3)), sftab, R, pmax);
     note_launch(1);
     return cudaGetLastError();
 }
 
 cudaError_t launch_pmax(const int *kept, const DevState *st, const double *zmin, const double *r2min, int p,
-                        long long n_obs, const double *sftab, double *pmax, int num_sms, cudaStream_t s) {
+                        long long n_obs, const double *sftab, const double *rt, double tau, double *pmax, int num_sms,
+                        cudaStream_t s) {
     const long long pairs = (long long)p * (p - 1) / 2;
     const long long want = (pairs + 255) / 256;
     const int blocks = (int)(want < (long long)num_sms * 2 ? want : (long long)num_sms * 2);
-    pmax_kept_kernel<<<blocks > 0 ? blocks : 1, 256, 0, s>>>(kept, st, zmin, r2min, sqrt((double)(n_obs - 3)), sftab,
+    const RTab R = rt_params(n_obs, tau, pairs, rt);
+    pmax_kept_kernel<<<blocks > 0 ? blocks : 1, 256, 0, s>>>(kept, st, zmin, r2min, sqrt((double)(n_obs - 3)), sftab, R,
                                                              pmax);
     note_launch(1);
     return cudaGetLastError();

@@ -54,6 +54,7 @@ struct BInst {
     long long n_obs;
     int p, n_thr;
     double sqrt_nm3;
+    RTab rt;              // pmax by |rho| (its table in this plan's workspace)
     double tau[BATCH_MAX_LEVEL + 1], t2[BATCH_MAX_LEVEL + 1];
     float t2lo[BATCH_MAX_LEVEL + 1], t2hi[BATCH_MAX_LEVEL + 1];
     L0Bounds l0;
@@ -265,11 +266,9 @@ __device__ __forceinline__ int inst_of(const long long *__restrict__ off, int co
 __device__ __forceinline__ bool skip_inst(const BInst &I, bool rerun) { return rerun && *(volatile int *)I.flag == 0; }
 
 // Per p^2 chunk: r2min = 1.4e306 (above every stored rho^2); chunk 0 also clears the
-// instance's DevState (and, on the first pass, its flag); block 0 builds the erfc
-// table of the pmax kernels.
+// instance's DevState (and, on the first pass, its flag).
 __global__ void batch_init_kernel(const BInst *__restrict__ inst, const long long *__restrict__ off_p2, int count,
-                                  double *__restrict__ sftab, bool rerun) {
-    if (blockIdx.x == 0 && !rerun) sf_table_build(reinterpret_cast<double (*)[SF_TERMS]>(sftab));  // erfc table for pmax
+                                  bool rerun) {
     long long lb;
     const BInst &I = inst[inst_of(off_p2, count, blockIdx.x, lb)];
     if (skip_inst(I, rerun)) return;
@@ -429,13 +428,15 @@ __global__ void __launch_bounds__(256, (L <= 2 ? 3 : 1)) batch_level_kernel(cons
 }
 
 // pmax of the pairs removed at level 0 and the -1 fill, per p^2 chunk.
-__global__ void batch_pmax_removed_kernel(const BInst *__restrict__ inst, const long long *__restrict__ off_p2,
-                                          int count, const double *__restrict__ sftab, bool rerun) {
-    __shared__ double tab[SF_CENTRES][SF_TERMS];
+__global__ void __launch_bounds__(256) batch_pmax_removed_kernel(const BInst *__restrict__ inst,
+                                                                 const long long *__restrict__ off_p2, int count,
+                                                                 const double *__restrict__ sftab, bool rerun) {
+    __shared__ PmaxShared S;
     long long lb;
     const BInst &I = inst[inst_of(off_p2, count, blockIdx.x, lb)];
     if (skip_inst(I, rerun)) return;  // uniform over the block
-    sf_table_load(tab, sftab);
+    const RTab R = I.rt;
+    pmax_tables_load(S, sftab, R);
     __syncthreads();
     const unsigned p = (unsigned)I.p;
     const unsigned total = p * p;
@@ -443,30 +444,39 @@ __global__ void batch_pmax_removed_kernel(const BInst *__restrict__ inst, const 
     for (unsigned k = k0 + threadIdx.x; k < k1; k += blockDim.x) {
         const unsigned i = k / p, j = k - i * p;
         if (i >= j) I.pmax[k] = -1.0;
-        else if (I.zmin[k] < 0.0) I.pmax[k] = two_sf_tab(I.sqrt_nm3 * fisher_z(I.C[k]), tab);
+        else if (I.zmin[k] < 0.0) I.pmax[k] = pmax_removed(S, R, I.sqrt_nm3, I.C[k]);
     }
 }
 
-// pmax of the pairs kept at level 0, block per instance.
-__global__ void batch_pmax_kept_kernel(const BInst *__restrict__ inst, const double *__restrict__ sftab, bool rerun) {
-    __shared__ double tab[SF_CENTRES][SF_TERMS];
-    const BInst &I = inst[blockIdx.x];
+// pmax of the pairs kept at level 0, BATCH_KEPT_BLOCKS blocks per instance (one block took
+// 410 us for 24 instances, most SMs idle, and 800 us for 256).
+constexpr int BATCH_KEPT_BLOCKS = 8;
+__global__ void __launch_bounds__(256) batch_pmax_kept_kernel(const BInst *__restrict__ inst,
+                                                              const double *__restrict__ sftab, bool rerun) {
+    __shared__ PmaxShared S;
+    const int b = (int)(blockIdx.x % BATCH_KEPT_BLOCKS);
+    const BInst &I = inst[blockIdx.x / BATCH_KEPT_BLOCKS];
     if (skip_inst(I, rerun)) return;  // uniform over the block
-    sf_table_load(tab, sftab);
-    __syncthreads();
     const int n = I.st->n_kept;
-    for (int t = threadIdx.x; t < n; t += blockDim.x) {
-        const int k = I.kept[t];
-        double z = I.zmin[k];
-        const double r2 = I.r2min[k];
-        if (r2 < 1.0) z = fmin(z, fisher_z(sqrt(r2)));
-        I.pmax[k] = two_sf_tab(I.sqrt_nm3 * z, tab);
-    }
+    if (b * (int)blockDim.x >= n) return;
+    const RTab R = I.rt;
+    pmax_tables_load(S, sftab, R);
+    __syncthreads();
+    pmax_kept_share(S, R, I.kept, n, I.zmin, I.r2min, I.sqrt_nm3, I.pmax, b, BATCH_KEPT_BLOCKS);
 }
 
-// The erfc table of the pmax kernels (a plan whose step finishes without its own init).
-__global__ void batch_sftab_kernel(double *__restrict__ sftab) {
-    sf_table_build(reinterpret_cast<double (*)[SF_TERMS]>(sftab));
+// The tables of the pmax kernels: block 0 the erfc table, then two blocks per instance for
+// its table of pmax by |rho| (rt: RT_CENTRES x RT_TERMS doubles each).
+__global__ void __launch_bounds__(RT_CENTRES / 2) batch_sftab_kernel(const BInst *__restrict__ inst,
+                                                                     double *__restrict__ sftab,
+                                                                     double *__restrict__ rt) {
+    if (blockIdx.x == 0) {
+        sf_table_build(reinterpret_cast<double (*)[SF_TERMS]>(sftab));
+        return;
+    }
+    const int k = ((int)blockIdx.x - 1) / 2, m = (((int)blockIdx.x - 1) & 1) * (RT_CENTRES / 2) + threadIdx.x;
+    const RTab R = inst[k].rt;
+    if (R.a != nullptr) rt_build(R, m, rt + ((size_t)k * RT_CENTRES + m) * RT_TERMS);
 }
 
 // [done, last level run, status, record ints] per instance.
@@ -486,7 +496,7 @@ namespace host {
 namespace {
 
 struct BatchLayout {
-    size_t table, off_tiles, off_rows, off_p2, edges, edge_off, sftab, flags, status, slices, total;
+    size_t table, off_tiles, off_rows, off_p2, edges, edge_off, sftab, rt, flags, status, slices, total;
 };
 
 size_t al(size_t x) { return (x + 255) / 256 * 256; }
@@ -515,6 +525,8 @@ BatchLayout layout(const int *p, int count) {
     off += al(((size_t)count + 1) * sizeof(long long));
     L.sftab = off;
     off += al((size_t)SF_CENTRES * SF_TERMS * sizeof(double));
+    L.rt = off;
+    off += al((size_t)count * RT_CENTRES * RT_TERMS * sizeof(double));
     L.flags = off;
     off += al((size_t)count * sizeof(int));
     L.status = off;
@@ -620,6 +632,10 @@ int build_header(const gcsl_gauss_instance *in, int count, int max_level, int pr
                 I.t2hi[l] = std::nextafter((float)(hi * hi), 2.0f);
             }
         }
+        double tau_max = 0.0;
+        for (int l = 0; l <= max_level; ++l) tau_max = std::max(tau_max, I.tau[l]);
+        I.rt = rt_params(X.n_obs, tau_max, (long long)p * (p - 1) / 2,
+                         reinterpret_cast<double *>(base + Ly.rt) + (size_t)k * RT_CENTRES * RT_TERMS);
         const long long nb = (p + 31) / 32;
         ot[k + 1] = ot[k] + nb * (nb + 1) / 2;
         orow[k + 1] = orow[k] + p;
@@ -730,10 +746,10 @@ int gauss_batch_step(const long long *plan, int first, int last, bool finish, bo
     const long long *op2 = reinterpret_cast<const long long *>(base + Ly.off_p2);
     long long *edges = reinterpret_cast<long long *>(base + Ly.edges);
     long long *eoff = reinterpret_cast<long long *>(base + Ly.edge_off);
-    double *sftab = reinterpret_cast<double *>(base + Ly.sftab);
+    double *sftab = reinterpret_cast<double *>(base + Ly.sftab), *rt = reinterpret_cast<double *>(base + Ly.rt);
 
     if (first == 0) {
-        batch_init_kernel<<<(unsigned)plan[PW_P2], 256, 0, s>>>(inst, op2, count, sftab, rerun);
+        batch_init_kernel<<<(unsigned)plan[PW_P2], 256, 0, s>>>(inst, op2, count, rerun);
         batch_level0_kernel<<<(unsigned)plan[PW_TILES], 256, 0, s>>>(inst, ot, count, rerun);
         note_launch(2);
     }
@@ -750,12 +766,12 @@ int gauss_batch_step(const long long *plan, int first, int last, bool finish, bo
         if (e != cudaSuccess) return GCSL_ERR_DEVICE;
     }
     if (finish) {
-        if (first != 0) {  // the erfc table of this plan's header is built by its init kernel
-            batch_sftab_kernel<<<1, 32, 0, s>>>(sftab);
+        if (!rerun) {  // a rerun finds the tables of the first pass
+            batch_sftab_kernel<<<1 + 2 * count, RT_CENTRES / 2, 0, s>>>(inst, sftab, rt);
             note_launch(1);
         }
         batch_pmax_removed_kernel<<<(unsigned)plan[PW_P2], 256, 0, s>>>(inst, op2, count, sftab, rerun);
-        batch_pmax_kept_kernel<<<count, 256, 0, s>>>(inst, sftab, rerun);
+        batch_pmax_kept_kernel<<<count * BATCH_KEPT_BLOCKS, 256, 0, s>>>(inst, sftab, rerun);
         note_launch(2);
     }
     if (host_status != nullptr) {

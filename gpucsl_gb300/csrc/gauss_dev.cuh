@@ -3,6 +3,8 @@
 // key bookkeeping of a level, the sepset write-back and the p-value functions.
 #pragma once
 
+#include <cmath>
+
 #include "common.cuh"
 
 namespace gcsl {
@@ -941,6 +943,148 @@ __device__ __forceinline__ double fisher_z(double r) {
         return fabs(r) * s;
     }
     return fabs(0.5 * log(fabs((1.0 + r) / (1.0 - r))));
+}
+
+// pmax of a pair straight from |rho|: f(r) = erfc(c atanh r), c = sqrt((n - 3) / 2), by Taylor
+// expansions about RT_CENTRES equidistant centres r = m w on [0, rmax].  Evaluating Z and
+// erfc one after the other takes about 36 FP64 operations a pair, this 10 -- on a pipe of
+// 1/64 of the FP32 rate they are the time of the pmax kernels.  rmax covers the pairs that a
+// test removed (|rho| below tanh of the largest threshold); the others, |rho| >= 1 and exact Z
+// minima take the evaluation above.  With c atanh(rmax) <= 3 and rmax <= 1/2 (rt_params) eight
+// terms leave a truncation below 6e-17 of the value; against 40 digits the error is below
+// 3e-15 relative over n = 30 .. 50000 and alpha = 2.5e-5 .. 0.05, smaller than that of the
+// two-step evaluation everywhere (it does not round the argument of erfc).
+constexpr int RT_CENTRES = 256, RT_TERMS = 8;
+constexpr int RT_STRIDE = RT_TERMS + 1;  // in shared memory: lanes at different centres meet different banks
+
+struct RTab {
+    const double *a;          // RT_CENTRES x RT_TERMS coefficients in global memory, or null: not used
+    double w, inv_w, rmax, rmax2;
+    double c;
+};
+
+// The table's parameters for n observations and largest threshold tau; a stays null where
+// the table does not hold (or does not pay: building it costs about as much as 3000 pairs).
+__host__ inline RTab rt_params(long long n_obs, double tau, long long pairs, const double *a) {
+    RTab R;
+    R.a = nullptr;
+    R.c = std::sqrt(0.5 * (double)(n_obs - 3));
+    R.rmax = std::tanh(tau) * (1.0 + 1e-6);
+    R.rmax2 = R.rmax * R.rmax * (1.0 - 1e-12);
+    R.w = R.rmax / (RT_CENTRES - 1);
+    R.inv_w = R.w > 0.0 ? 1.0 / R.w : 0.0;
+    const bool ok = pairs >= 8192 && tau > 0.0 && R.rmax <= 0.5 && R.c * std::atanh(R.rmax) <= 3.0;  // false for NaN
+    if (ok) R.a = a;
+    return R;
+}
+
+// Coefficients of centre m: power series (in t = r - r0) of q = c / (1 - r^2), g = c atanh r
+// (g' = q), E = exp(-g^2) (E' = -2 g q E) and f' = -(2 / sqrt pi) q E.
+__device__ __forceinline__ void rt_build(const RTab &R, int m, double *__restrict__ out) {
+    const double r0 = m * R.w, ih = 1.0 / (1.0 - r0 * r0);
+    double q[RT_TERMS - 1], g[RT_TERMS - 1], u[RT_TERMS - 1], E[RT_TERMS - 1];
+    q[0] = R.c * ih;
+    q[1] = 2.0 * r0 * q[0] * ih;
+#pragma unroll
+    for (int k = 2; k < RT_TERMS - 1; ++k) q[k] = fma(2.0 * r0, q[k - 1], q[k - 2]) * ih;
+    g[0] = R.c * atanh(r0);
+#pragma unroll
+    for (int k = 0; k + 1 < RT_TERMS - 1; ++k) g[k + 1] = q[k] * (1.0 / (k + 1));
+#pragma unroll
+    for (int k = 0; k < RT_TERMS - 1; ++k) {
+        u[k] = 0.0;
+#pragma unroll
+        for (int j = 0; j <= k; ++j) u[k] = fma(g[j], q[k - j], u[k]);
+    }
+    E[0] = exp(-g[0] * g[0]);
+    out[0] = erfc(g[0]);
+#pragma unroll
+    for (int k = 0; k < RT_TERMS - 1; ++k) {
+        double e = 0.0, f = 0.0;
+#pragma unroll
+        for (int j = 0; j <= k; ++j) {
+            e = fma(u[j], E[k - j], e);
+            f = fma(q[j], E[k - j], f);
+        }
+        if (k + 1 < RT_TERMS - 1) E[k + 1] = -2.0 / (k + 1) * e;
+        out[k + 1] = -1.12837916709551257390 / (k + 1) * f;  // 2 / sqrt(pi)
+    }
+}
+
+// The table into a block's shared memory (RT_CENTRES * RT_STRIDE doubles).
+__device__ __forceinline__ void rt_load(double *__restrict__ sm, const double *__restrict__ a) {
+    for (int k = threadIdx.x; k < RT_CENTRES * RT_TERMS; k += blockDim.x)
+        sm[(k / RT_TERMS) * RT_STRIDE + k % RT_TERMS] = __ldg(a + k);
+}
+
+// f(r) for 0 <= r < rmax: the nearest centre by adding 1.5 * 2^52 (the sum's low bits are the
+// rounded quotient), then Horner.
+__device__ __forceinline__ double rt_eval(const RTab &R, const double *__restrict__ sm, double r) {
+    constexpr double magic = 6755399441055744.0;
+    const double v = fma(r, R.inv_w, magic);
+    const unsigned m = min((unsigned)__double_as_longlong(v), (unsigned)(RT_CENTRES - 1));
+    const double t = fma(-(v - magic), R.w, r);
+    const double *a = sm + m * RT_STRIDE;
+    double f = a[RT_TERMS - 1];
+#pragma unroll
+    for (int k = RT_TERMS - 2; k >= 0; --k) f = fma(f, t, a[k]);
+    return f;
+}
+
+// Shared memory of the pmax kernels.
+struct PmaxShared {
+    double sf[SF_CENTRES][SF_TERMS];
+    double rt[RT_CENTRES * RT_STRIDE];
+};
+__device__ __forceinline__ void pmax_tables_load(PmaxShared &S, const double *__restrict__ sftab, const RTab &R) {
+    sf_table_load(S.sf, sftab);
+    if (R.a != nullptr) rt_load(S.rt, R.a);
+}
+
+// pmax of a pair removed at level 0, from its correlation.
+__device__ __forceinline__ double pmax_removed(const PmaxShared &S, const RTab &R, double sqrt_nm3, double c) {
+    const double r = fabs(c);
+    if (R.a != nullptr && r < R.rmax) return rt_eval(R, S.rt, r);
+    return two_sf_tab(sqrt_nm3 * fisher_z(c), S.sf);
+}
+
+// pmax of the pairs kept at level 0, share b of nb blocks of 256 threads: z* = min(zmin, Z of
+// the smallest rho^2 any later level stored), pmax = 2 sf(sqrt(n - 3) z*) (helpers.py:62-82
+// with the FP64 z*).  Pairs that a later level removed have a small rho^2 and take the table;
+// the others are queued and evaluated densely (a warp would otherwise run the long evaluation
+// for the few lanes that need it in every round).
+constexpr int PMAX_QUEUE = 1024;
+__device__ __forceinline__ void pmax_kept_share(const PmaxShared &S, const RTab &R, const int *__restrict__ kept, int n,
+                                                const double *__restrict__ zmin, const double *__restrict__ r2min,
+                                                double sqrt_nm3, double *__restrict__ pmax, int b, int nb) {
+    __shared__ int s_queue[PMAX_QUEUE];
+    __shared__ int s_n;
+    const double inf = __longlong_as_double(0x7ff0000000000000ll);
+    if (threadIdx.x == 0) s_n = 0;
+    __syncthreads();
+    for (int t0 = b * blockDim.x; t0 < n; t0 += nb * blockDim.x) {
+        const int t = t0 + threadIdx.x;
+        if (t < n) {
+            const int k = kept[t];
+            const double r2 = r2min[k];
+            if (R.a != nullptr && r2 < R.rmax2 && zmin[k] == inf) pmax[k] = rt_eval(R, S.rt, sqrt(r2));
+            else s_queue[atomicAdd(&s_n, 1)] = k;
+        }
+        __syncthreads();
+        const int queued = s_n;
+        if (queued + (int)blockDim.x > PMAX_QUEUE || t0 + nb * (int)blockDim.x >= n) {  // full, or the last round
+            for (int q = threadIdx.x; q < queued; q += blockDim.x) {
+                const int k = s_queue[q];
+                double z = zmin[k];
+                const double r2 = r2min[k];
+                if (r2 < 1.0) z = fmin(z, fisher_z(sqrt(r2)));  // Z increasing in rho^2 below 1
+                pmax[k] = two_sf_tab(sqrt_nm3 * z, S.sf);
+            }
+            __syncthreads();
+            if (threadIdx.x == 0) s_n = 0;
+            __syncthreads();
+        }
+    }
 }
 
 }  // namespace gcsl
