@@ -490,13 +490,37 @@ __global__ void batch_status_kernel(const BInst *__restrict__ inst, int count, i
     out[4 * k + 3] = (int)*(volatile const unsigned long long *)&st->n_rec_ints;
 }
 
+// What collect reports of an instance, so that one copy brings all of them to the host (a
+// copy of each DevState took 8 us apiece).
+struct BatchReport {
+    int status, last_level, rerun, pad;
+    long long n_rec_ints, tests, retests;
+};
+
+__global__ void batch_report_kernel(const BInst *__restrict__ inst, int count, BatchReport *__restrict__ out) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= count) return;
+    const BInst &I = inst[k];
+    const DevState *st = I.st;
+    BatchReport r;
+    r.status = st->status;
+    r.last_level = st->last_level;
+    r.rerun = *I.flag != 0 ? 1 : 0;
+    r.pad = 0;
+    r.n_rec_ints = (long long)st->n_rec_ints;
+    r.retests = (long long)st->retests;
+    r.tests = (long long)I.p * (I.p - 1) / 2;
+    for (int l = 1; l <= BATCH_MAX_LEVEL; ++l) r.tests += (long long)st->tests[l];
+    out[k] = r;
+}
+
 // ---------------------------------------------------------------------- host
 namespace host {
 
 namespace {
 
 struct BatchLayout {
-    size_t table, off_tiles, off_rows, off_p2, edges, edge_off, sftab, rt, flags, status, slices, total;
+    size_t table, off_tiles, off_rows, off_p2, edges, edge_off, sftab, rt, flags, status, report, slices, total;
 };
 
 size_t al(size_t x) { return (x + 255) / 256 * 256; }
@@ -531,6 +555,8 @@ BatchLayout layout(const int *p, int count) {
     off += al((size_t)count * sizeof(int));
     L.status = off;
     off += al((size_t)count * 4 * sizeof(int));
+    L.report = off;
+    off += al((size_t)count * sizeof(BatchReport));
     L.slices = off;
     if (p)  // p == nullptr: every instance brings its own state slice
         for (int k = 0; k < count; ++k) off += slice_bytes(p[k]);
@@ -793,36 +819,29 @@ int gauss_batch_run(const long long *plan, cudaStream_t s, bool rerun) {
     return gauss_batch_step(plan, 0, (int)plan[PW_MAXL], true, rerun, nullptr, s);
 }
 
-// Synchronises the stream and copies every instance's state back into the outputs.
+// Gathers every instance's state, synchronises the stream and fills the outputs.
 int gauss_batch_collect(const long long *plan, gcsl_gauss_instance *out, int count, cudaStream_t s) {
     if (!gauss_batch_plan_ok(plan) || count != (int)plan[PW_COUNT]) return GCSL_ERR_INVALID_ARG;
     char *base = reinterpret_cast<char *>(static_cast<uintptr_t>(plan[PW_WS]));
-    std::vector<BInst> tab((size_t)count);
-    if (cudaMemcpyAsync(tab.data(), base, tab.size() * sizeof(BInst), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+    const BatchLayout Ly = layout(nullptr, count);
+    BatchReport *dev = reinterpret_cast<BatchReport *>(base + Ly.report);
+    batch_report_kernel<<<(count + 127) / 128, 128, 0, s>>>(reinterpret_cast<const BInst *>(base + Ly.table), count, dev);
+    note_launch(1);
+    std::vector<BatchReport> rep((size_t)count);
+    if (cudaGetLastError() != cudaSuccess ||
+        cudaMemcpyAsync(rep.data(), dev, rep.size() * sizeof(BatchReport), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
         cudaStreamSynchronize(s) != cudaSuccess)
         return GCSL_ERR_DEVICE;
-    std::vector<int> flags((size_t)count, 0);
-    if (cudaMemcpyAsync(flags.data(), gauss_batch_flags(plan), (size_t)count * sizeof(int), cudaMemcpyDeviceToHost,
-                        s) != cudaSuccess)
-        return GCSL_ERR_DEVICE;
-    std::vector<DevState> st((size_t)count);
-    for (int k = 0; k < count; ++k)
-        if (cudaMemcpyAsync(&st[(size_t)k], tab[(size_t)k].st, sizeof(DevState), cudaMemcpyDeviceToHost, s) !=
-            cudaSuccess)
-            return GCSL_ERR_DEVICE;
-    if (cudaStreamSynchronize(s) != cudaSuccess) return GCSL_ERR_DEVICE;
     int first = GCSL_OK;
     for (int k = 0; k < count; ++k) {
-        const DevState &h = st[(size_t)k];
+        const BatchReport &h = rep[(size_t)k];
         gcsl_gauss_instance &o = out[k];
         o.status = h.status;
         o.levels_run = h.last_level + 1;
         o.n_records = (int64_t)h.n_rec_ints;
-        long long tests = (long long)o.p * (o.p - 1) / 2;
-        for (int l = 1; l <= BATCH_MAX_LEVEL; ++l) tests += (long long)h.tests[l];
-        o.tests = tests;
+        o.tests = h.tests;
         o.retests = (int64_t)h.retests;
-        o.exact_rerun = flags[(size_t)k] != 0 ? 1 : 0;
+        o.exact_rerun = h.rerun;
         if (first == GCSL_OK && h.status != GCSL_OK) first = h.status;
     }
     return first;
