@@ -9,10 +9,10 @@
 //  2. split I = sum_k d_k 2^(7 (6 - k)), k = 0..6, into signed 7-bit digits
 //     (|d_0| <= 128, |d_k| <= 64): every digit is exact in BF16;
 //  3. for each digit pair with k + l = g <= 6 accumulate d_k^T d_l on the tensor core
-//     into accumulator g (FP32 in TMEM).  Products are at most 2^14 and a group sums at
-//     most (g + 3) 2^12 per sample, so over 448 samples every partial sum stays below
-//     2^24: the FP32 accumulators hold exact integers;
-//  4. every 448 samples the 7 accumulators are drained into two int64 words per output
+//     into accumulator g (FP32 in TMEM).  While every partial sum stays at most 2^24 the FP32
+//     accumulators hold exact integers: 448 samples always, about 1600 for Gaussian columns
+//     (chunk_steps below takes the number from the data);
+//  4. at the end of each such chunk the 7 accumulators are drained into two int64 words per output
 //     (groups 0-2 weighted 2^14, 2^7, 1 and groups 3-6 weighted 2^21 .. 1); split-K
 //     partial words are summed exactly, and the value 2^28 hi + lo is rounded to FP64
 //     once.
@@ -45,7 +45,8 @@ constexpr int OZ_S = 7;                 // digits per value (all written by the 
 constexpr int OZ_S_SPLIT = 5;           // digits of the split-precision product
 constexpr int OZ_TM = 128, OZ_TN = 64;  // output tile
 constexpr int OZ_KS = 32;               // sample padding granule
-constexpr int OZ_CHUNK_STEPS = 28;      // 448 samples (28 MMA K steps) between exact drains
+constexpr int OZ_WINDOW_STEPS = 4;      // 64 samples (K steps of 16): the windows of the energy bound
+constexpr int OZ_MIN_WINDOWS = 7, OZ_MAX_WINDOWS = 64;  // windows between exact drains (chunk_steps)
 constexpr uint32_t OZ_TMEM_COLS = 512;
 // shared-memory bytes of one K step for NS digits: NS x (128 A rows + 64 B rows) x 16
 // samples x 2 bytes (NS = 7: 28672 + 14336)
@@ -73,6 +74,7 @@ struct OzJob {
     double *partial, *mean, *inv_sd;
     long long *kmin, *kmax;
     int *expo, *err;
+    unsigned *energy;  // largest digit energy of a column over a window
     uint8_t *dig;
     long long *phi, *plo;
     double *C;
@@ -158,6 +160,7 @@ __global__ void colstats_init_kernel(Src src) {
         J.kmax[j] = (long long)0x8000000000000000ull;
         if (j == 0) {
             *J.err = 0;
+            *J.energy = 0u;
             double *slot = src.err_slot(J.index);
             if (slot != nullptr) *slot = 0.0;
         }
@@ -282,9 +285,21 @@ __global__ void col_mean_exp_kernel(Src src) {
 // One block covers 32 columns x 64 samples: lane = column, warp = group of 8 consecutive
 // samples, so a thread owns one 16-byte row of a core matrix per digit (8 samples of one
 // column).  It loads its 8 samples (each load a coalesced row of 32 columns), splits
-// them, packs each digit's 8 BF16 values and stores the 16 bytes: no shared memory and
-// no barrier.
-constexpr int OZ_DIG_SAMPLES = 64;  // samples per digit-split block
+// them, packs each digit's 8 BF16 values and stores the 16 bytes.
+//
+// Digits are rounded half up from the highest down.  That makes d_k the k-th 7-bit field of I
+// in two's complement plus the top bit of the field below it, so all digits of a value come
+// from a few shifts: 64 + d_k as bytes b of two words, and BF16 as the bits 0x4300 + b
+// (128 + b) less 192, two samples to an instruction.  Digit by digit with shifts and
+// subtractions the kernel was bound by the integer pipe.
+constexpr int OZ_DIG_SAMPLES = 64;  // samples per digit-split block: one window of the energy bound
+
+// (a - c, b - c) of packed BF16 pairs.
+__device__ __forceinline__ uint32_t bf162_sub(uint32_t a, uint32_t c) {
+    uint32_t r;
+    asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(c));
+    return r;
+}
 
 // Two floats as one word of two BF16 values, lo in the low half (the lower address).
 __device__ __forceinline__ uint32_t bf16x2_rn(float lo, float hi) {
@@ -299,7 +314,7 @@ __host__ __device__ inline long long oz_digit_blocks(const OzDims &D) {
 }
 
 template <typename T, int NW>
-__device__ __forceinline__ void digit_split_block(const OzJob &Jb, long long lb) {
+__device__ __forceinline__ void digit_split_block(const OzJob &Jb, long long lb, unsigned (*s_energy)[32]) {
     const T *__restrict__ X = static_cast<const T *>(Jb.X);
     const long long n = Jb.n, ldx = Jb.ldx;
     const int p = Jb.p, p_pad = Jb.D.p_pad;
@@ -308,7 +323,6 @@ __device__ __forceinline__ void digit_split_block(const OzJob &Jb, long long lb)
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;  // 8 warps
     const long long tg = (lb % ntx) * OZ_DIG_SAMPLES + 8 * w;  // the thread's first sample
     const int j = (int)(lb / ntx) * 32 + lane;
-    if (tg >= n_pad) return;  // the last block of a column strip may cover only 32 samples (uniform per warp)
     const bool col = j < p;
     const double mu = col ? Jb.mean[j] : 0.0;
     const int ej = col ? Jb.expo[j] : 0;
@@ -318,8 +332,10 @@ __device__ __forceinline__ void digit_split_block(const OzJob &Jb, long long lb)
         const long long t = tg + e;
         x[e] = (col && t < n) ? (double)X[t * ldx + j] : 0.0;
     }
-    uint32_t wds[OZ_S][4];
-    float fe[OZ_S];  // the digits of the even sample of the current pair
+    // digit 0, and 64 + digit as bytes: digits 4, 3, 2, 1 (byte 0 up) and 6, 5
+    int d0[8];
+    uint32_t b_hi[8], b_lo[8];
+    unsigned energy = 0;
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
         long long I = 0;
@@ -336,61 +352,90 @@ __device__ __forceinline__ void digit_split_block(const OzJob &Jb, long long lb)
             if (sh < 63) mag = (m + (1ll << (sh - 1))) >> sh;
             I = bits < 0 ? -mag : mag;
         }
-        // digits by rounding half up (arithmetic shifts), in 32-bit arithmetic: with
-        // I = H 2^21 + Lo (0 <= Lo < 2^21, |H| <= 2^28) the first three digits (weights
-        // 2^42, 2^35, 2^28) round at 2^41, 2^34, 2^27, all above Lo, so they follow from
-        // H alone: d = floor((H + 2^(s-1)) / 2^s) for s = 21, 14, 7 with H reduced after
-        // each; the remainder H 2^21 + Lo is then below 2^27 in magnitude
-        int d[OZ_S];
-        int hi = (int)(I >> 21);
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            const int sh = 7 * (2 - k) + 7;  // 21, 14, 7
-            d[k] = (hi + (1 << (sh - 1))) >> sh;
-            hi -= d[k] * (1 << sh);
+        // fields 1 .. 4 of I spread to bytes, then (field ^ 64) plus the next field's top bit
+        const uint32_t f = (uint32_t)(I >> 14), low = (uint32_t)I;
+        const uint32_t sp = (f & 0x7fu) | ((f << 1) & 0x7f00u) | ((f << 2) & 0x7f0000u) | ((f << 3) & 0x7f000000u);
+        b_hi[e] = (sp ^ 0x40404040u) + (((sp << 2) & 0x01010100u) | ((low >> 13) & 1u));
+        d0[e] = (int)((I + (1ll << 41)) >> 42);
+        // the sum of squared digits: sum b^2 - 128 sum b + 64^2 each
+        unsigned sq = __dp4a(b_hi[e], b_hi[e], (unsigned)(d0[e] * d0[e]) + 4u * 4096u);
+        unsigned su = __dp4a(b_hi[e], 0x01010101u, 0u);
+        if (NW > OZ_S_SPLIT) {
+            const uint32_t s2 = (low & 0x7fu) | ((low << 1) & 0x7f00u);
+            b_lo[e] = (s2 ^ 0x4040u) + ((s2 << 2) & 0x0100u);
+            sq = __dp4a(b_lo[e], b_lo[e], sq + 2u * 4096u);
+            su = __dp4a(b_lo[e], 0x0101u, su);
         }
-        int rem32 = hi * (1 << 21) + (int)(I & 0x1fffff);
+        energy += sq - 128u * su;
+    }
+    // the columns' energies over the block's 64 samples
+    s_energy[w][lane] = energy;
+    __syncthreads();
+    if (w == 0) {
 #pragma unroll
-        for (int k = 3; k < OZ_S - 1; ++k) {
-            const int sh = 7 * (OZ_S - 1 - k);
-            d[k] = (rem32 + (1 << (sh - 1))) >> sh;
-            rem32 -= d[k] * (1 << sh);
-        }
-        d[OZ_S - 1] = rem32;
-        // small integers to float exactly by the 1.5 * 2^23 offset (an integer add and an
-        // FP32 subtraction); a digit (|d| <= 128) has at most 8 significant bits, so it is
-        // exact in BF16, and two samples' digits become one packed word by one conversion
+        for (int q = 1; q < 8; ++q) energy += s_energy[q][lane];
+        energy = __reduce_max_sync(GCSL_FULL_MASK, energy);
+        if (lane == 0 && energy > *(volatile unsigned *)Jb.energy) atomicMax(Jb.energy, energy);
+    }
+    if (tg < n_pad) {  // the last block of a column strip may cover only 32 samples (uniform per warp)
+        const int nI = p_pad / OZ_TM;
+        const long long nq = n_pad / 16;
+        uint8_t *__restrict__ dig = Jb.dig;
+        const size_t roff = tc::kmajor_offset((uint32_t)(j % OZ_TM), (uint32_t)(tg % 16));
 #pragma unroll
         for (int k = 0; k < NW; ++k) {
-            const float f = __int_as_float(0x4B400000 + d[k]) - 12582912.0f;
-            if (e & 1) wds[k][e >> 1] = bf16x2_rn(fe[k], f);
-            else fe[k] = f;
+            uint32_t wd[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int e = 2 * q;
+                if (k == 0) {  // -128 .. 128, exact in BF16
+                    wd[q] = bf16x2_rn(__int_as_float(0x4B400000 + d0[e]) - 12582912.0f,
+                                      __int_as_float(0x4B400000 + d0[e + 1]) - 12582912.0f);
+                } else {
+                    const int at = k <= 4 ? 4 - k : 6 - k;  // place of the digit in its word
+                    const uint32_t c = __byte_perm(k <= 4 ? b_hi[e] : b_lo[e], k <= 4 ? b_hi[e + 1] : b_lo[e + 1],
+                                                   (uint32_t)(at * 0x11 + (at + 4) * 0x1100));
+                    wd[q] = bf162_sub((c & 0x00ff00ffu) + 0x43004300u, 0x43404340u);
+                }
+            }
+            const size_t off = (((size_t)k * nI + j / OZ_TM) * nq + tg / 16) * 4096 + roff;
+            *reinterpret_cast<uint4 *>(dig + off) = make_uint4(wd[0], wd[1], wd[2], wd[3]);
         }
     }
-    const int nI = p_pad / OZ_TM;
-    const long long nq = n_pad / 16;
-    uint8_t *__restrict__ dig = Jb.dig;
-    const size_t roff = tc::kmajor_offset((uint32_t)(j % OZ_TM), (uint32_t)(tg % 16));
-#pragma unroll
-    for (int k = 0; k < NW; ++k) {
-        const size_t off = (((size_t)k * nI + j / OZ_TM) * nq + tg / 16) * 4096 + roff;
-        *reinterpret_cast<uint4 *>(dig + off) = make_uint4(wds[k][0], wds[k][1], wds[k][2], wds[k][3]);
-    }
+    __syncthreads();  // s_energy is reused by the next block of the range
+}
+
+// K steps between drains: the largest count whose partial sums surely stay at most 2^24.
+//
+// With W the largest sum of squared digits of any column over a window of 64 samples, a
+// chunk of b windows has |sum_t sum_{k + l = g} d_k,ti d_l,tj| <= half the two columns' digit
+// energies over the chunk (2 |a b| <= a^2 + b^2 for each product; a digit occurs once in a
+// group) <= b W.  Seven windows are always allowed: products are at most 2^14 and a group sums
+// at most (g + 3) 2^12 per sample, 9 * 2^12 * 448 < 2^24.
+//
+// A drain stalls the MMAs for about 2.3 us (57344 conversions at 16 a clock, one load after
+// another): 7 % of the time with 28 steps a chunk, 2 % with the 100 that Gaussian columns
+// allow (product at p = 1999, n = 49999).
+__device__ __forceinline__ int chunk_steps(unsigned W) {
+    const unsigned b = W > 0u ? (1u << 24) / W : (unsigned)OZ_MAX_WINDOWS;
+    return OZ_WINDOW_STEPS *
+           (int)(b < OZ_MIN_WINDOWS ? OZ_MIN_WINDOWS : b > (unsigned)OZ_MAX_WINDOWS ? OZ_MAX_WINDOWS : b);
 }
 
 template <typename T, class Src, int NW = OZ_S>
 __global__ void __launch_bounds__(256) digit_split_kernel(Src src, long long total) {
+    __shared__ unsigned s_energy[8][32];
     pdl_wait();
     pdl_trigger();
     if constexpr (std::is_same<Src, OneJob>::value) {
         (void)total;
-        digit_split_block<T, NW>(src.job, blockIdx.x);
+        digit_split_block<T, NW>(src.job, blockIdx.x, s_energy);
     } else {
         __shared__ OzJob s_job;
         __shared__ long long s_rng[2];
         stage_blocks(src, total, s_job, s_rng, [&](const OzJob &J, long long lb) {
             if (src.skip(J.index)) return;  // not selected in this run (uniform over the block)
-            digit_split_block<T, NW>(J, lb);
+            digit_split_block<T, NW>(J, lb, s_energy);
         });
     }
 }
@@ -400,11 +445,12 @@ __global__ void __launch_bounds__(256) digit_split_kernel(Src src, long long tot
 // only find their job unflagged).
 template <typename T>
 __global__ void digit_split_flagged_kernel(const OzJob *__restrict__ jobs, int count, const int *__restrict__ active) {
+    __shared__ unsigned s_energy[8][32];
     for (int k = 0; k < count; ++k) {
         if (active[k] == 0) continue;  // uniform over the block
         const OzJob J = jobs[k];
         const long long nb = oz_digit_blocks(J.D);
-        for (long long lb = blockIdx.x; lb < nb; lb += gridDim.x) digit_split_block<T, OZ_S>(J, lb);
+        for (long long lb = blockIdx.x; lb < nb; lb += gridDim.x) digit_split_block<T, OZ_S>(J, lb, s_energy);
     }
 }
 
@@ -520,7 +566,8 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     const long long nq = D.n_pad / 16;
     const long long q0 = (long long)split * D.slabs_per_split;
     const long long nst = min(q0 + (long long)D.slabs_per_split, nq) - q0;  // K steps of this split
-    const int nchunks = (int)((nst + OZ_CHUNK_STEPS - 1) / OZ_CHUNK_STEPS);
+    const int per_chunk = chunk_steps(*s_job.energy);
+    const int nchunks = (int)((nst + per_chunk - 1) / per_chunk);
 
     if (warp == 0) tc::tmem_alloc(&tmem_slot, OZ_TMEM_COLS);
     if (tid == 0) {
@@ -590,7 +637,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
                     break;
                 }
                 tc::fence_after_sync();
-                const long long c0 = (long long)c * OZ_CHUNK_STEPS, c1 = min(c0 + OZ_CHUNK_STEPS, nst);
+                const long long c0 = (long long)c * per_chunk, c1 = min(c0 + per_chunk, nst);
                 bool bad = false;
                 for (long long st = c0; st < c1; ++st) {
                     const int b = (int)(st % NST);
@@ -917,7 +964,8 @@ static OzDims oz_dims(long long n, int p, int num_sms, int splits_req = 0) {
     if (splits_req <= 0 && splits > (steps + OZ_MIN_STEPS - 1) / OZ_MIN_STEPS)
         splits = (int)((steps + OZ_MIN_STEPS - 1) / OZ_MIN_STEPS);
     if (splits > steps) splits = (int)steps;
-    D.slabs_per_split = (int)((steps + splits - 1) / splits);
+    // whole windows per split, so that a chunk's steps lie in the windows its bound counts
+    D.slabs_per_split = (int)((steps + splits - 1) / splits + OZ_WINDOW_STEPS - 1) / OZ_WINDOW_STEPS * OZ_WINDOW_STEPS;
     D.splits = (int)((steps + D.slabs_per_split - 1) / D.slabs_per_split);
     return D;
 }
@@ -954,6 +1002,7 @@ static size_t oz_job(OzJob &J, void *ws, const void *X, long long n, int p, long
     J.kmax = reinterpret_cast<long long *>(take((size_t)p * sizeof(long long)));
     J.expo = reinterpret_cast<int *>(take((size_t)p * sizeof(int)));
     J.err = reinterpret_cast<int *>(take(sizeof(int)));
+    J.energy = reinterpret_cast<unsigned *>(take(sizeof(unsigned)));
     J.dig = reinterpret_cast<uint8_t *>(take((size_t)OZ_S * D.p_pad * (size_t)D.n_pad * sizeof(uint16_t)));
     J.phi = reinterpret_cast<long long *>(take((size_t)D.splits * D.p_pad * (size_t)D.p_pad * sizeof(long long) * 2));
     J.plo = J.phi ? J.phi + (size_t)D.splits * D.p_pad * (size_t)D.p_pad : nullptr;
