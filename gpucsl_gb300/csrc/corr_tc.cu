@@ -148,6 +148,52 @@ __device__ __forceinline__ double key_value(long long k) {
 
 constexpr int OZ_STAT_ROWS = 512;  // samples per column-statistics block
 
+// A float widened to FP64 on its bits: the conversion instruction runs on the FP64 pipe (1/64
+// of the FP32 rate), which bounds the kernels that read every sample.  Right for zero and
+// normal floats; `odd` is set for the others (subnormal, infinite, NaN).  One branch covers
+// eight samples: a test per sample cost the digit kernel more than the conversions did.
+// n = 49999, p = 1999: column statistics 379 -> 207 us (with eight loads in flight and 32-bit
+// keys), digits 487 -> 401 us.
+__device__ __forceinline__ double widen_bits(float x, bool &odd) {
+    const unsigned u = __float_as_uint(x), m = u & 0x7fffffffu;
+    odd |= m != 0u && m - 0x00800000u >= 0x7f000000u;
+    const unsigned hi = m != 0u ? (m >> 3) + 0x38000000u : 0u;
+    return __hiloint2double((int)((u & 0x80000000u) | hi), (int)(u << 29));
+}
+// N samples in FP64, the odd ones among them by the conversion instruction.
+template <int N>
+__device__ __forceinline__ void samples_f64(const double (&x)[N], double (&y)[N]) {
+#pragma unroll
+    for (int e = 0; e < N; ++e) y[e] = x[e];
+}
+template <int N>
+__device__ __forceinline__ void samples_f64(const float (&x)[N], double (&y)[N]) {
+    bool odd = false;
+#pragma unroll
+    for (int e = 0; e < N; ++e) y[e] = widen_bits(x[e], odd);
+    if (odd) {
+#pragma unroll 1
+        for (int e = 0; e < N; ++e) {
+            const double v = (double)x[e];
+#pragma unroll
+            for (int q = 0; q < N; ++q)
+                if (q == e) y[q] = v;
+        }
+    }
+}
+
+// Order-preserving key of a sample for its minimum and maximum (a float's fits 32 bits), and
+// the key of its FP64 value.
+__device__ __forceinline__ long long sample_key(double x) { return ordered_key(x); }
+__device__ __forceinline__ int sample_key(float x) {
+    const int k = __float_as_int(x);
+    return k < 0 ? (k ^ 0x7fffffff) : k;
+}
+__device__ __forceinline__ long long widen_key(long long k) { return k; }
+__device__ __forceinline__ long long widen_key(int k) {
+    return ordered_key((double)__int_as_float(k < 0 ? (k ^ 0x7fffffff) : k));
+}
+
 template <class Src>
 __global__ void colstats_init_kernel(Src src) {
     pdl_wait();
@@ -207,17 +253,39 @@ __device__ __forceinline__ void colstats_block(const OzJob &Jb, long long lb, do
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int j = bx * 32 + lane;
     const long long t0 = (long long)by * OZ_STAT_ROWS, t1 = min(n, t0 + OZ_STAT_ROWS);
+    // eight samples' loads in flight; a column's sum keeps the order of its samples
+    using Key = decltype(sample_key(T(0)));
     double sum = 0.0;
-    long long mn = 0x7fffffffffffffffll, mx = (long long)0x8000000000000000ull;
-    if (j < p) {
-        for (long long t = t0 + w; t < t1; t += 8) {
-            const double x = (double)X[t * ldx + j];
-            sum += x;
-            const long long k = ordered_key(x);
-            mn = k < mn ? k : mn;
-            mx = k > mx ? k : mx;
+    Key kmn = 0, kmx = 0;
+    bool any = false;
+    if (j < p && t0 + w < t1) {
+        any = true;
+        kmn = kmx = sample_key(X[(t0 + w) * ldx + j]);
+        long long t = t0 + w;
+        for (; t + 56 < t1; t += 64) {
+            T x[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) x[e] = X[(t + 8 * e) * ldx + j];
+            double y[8];
+            samples_f64<8>(x, y);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                sum += y[e];
+                const Key k = sample_key(x[e]);
+                kmn = k < kmn ? k : kmn;
+                kmx = k > kmx ? k : kmx;
+            }
+        }
+        for (; t < t1; t += 8) {
+            const T x = X[t * ldx + j];
+            sum += (double)x;
+            const Key k = sample_key(x);
+            kmn = k < kmn ? k : kmn;
+            kmx = k > kmx ? k : kmx;
         }
     }
+    long long mn = any ? widen_key(kmn) : 0x7fffffffffffffffll;
+    long long mx = any ? widen_key(kmx) : (long long)0x8000000000000000ull;
     ssum[w][lane] = sum;
     smin[w][lane] = mn;
     smax[w][lane] = mx;
@@ -326,12 +394,11 @@ __device__ __forceinline__ void digit_split_block(const OzJob &Jb, long long lb,
     const bool col = j < p;
     const double mu = col ? Jb.mean[j] : 0.0;
     const int ej = col ? Jb.expo[j] : 0;
-    double x[8];
+    T raw[8];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-        const long long t = tg + e;
-        x[e] = (col && t < n) ? (double)X[t * ldx + j] : 0.0;
-    }
+    for (int e = 0; e < 8; ++e) raw[e] = (col && tg + e < n) ? X[(tg + e) * ldx + j] : T(0);
+    double x[8];
+    samples_f64<8>(raw, x);
     // digit 0, and 64 + digit as bytes: digits 4, 3, 2, 1 (byte 0 up) and 6, 5
     int d0[8];
     uint32_t b_hi[8], b_lo[8];

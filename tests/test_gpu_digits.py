@@ -60,3 +60,20 @@ def test_batch_equals_single(cuda):
     b.run()
     for k, X in enumerate(Xs):
         assert cuda.equal(b.C[k], engine.correlation(X))
+
+
+@pytest.mark.parametrize("n,p", [(9, 5), (64, 33), (577, 65), (1531, 40)])
+def test_floats_widen_exactly(cuda, n, p):
+    """FP32 samples with zeros, subnormals and the largest finite values give the bits of the
+    same samples held in FP64."""
+    from gpucsl_gb300 import engine
+
+    rng = np.random.default_rng(n + p)
+    X = (rng.standard_normal((n, p)) * 10.0 ** rng.integers(-30, 30, p)).astype(np.float32)
+    odd = np.array([0.0, -0.0, 1e-45, -1e-45, 1.1e-38, -1.1e-38, 1.1754944e-38, 3.4e38, -3.4e38], np.float32)
+    hit = rng.random((n, p)) < 0.05
+    X[hit] = rng.choice(odd, int(hit.sum()))
+    X[:, 0] = (rng.integers(-3, 4, n) * np.float32(1e-45)).astype(np.float32)  # subnormal throughout
+    X[0, 0] = np.float32(5e-45)
+    x32 = cuda.from_numpy(X).cuda()
+    assert cuda.equal(engine.correlation(x32), engine.correlation(cuda.from_numpy(X.astype(np.float64)).cuda()))
