@@ -264,7 +264,9 @@ def ordinal_encode_device(X, ld: int | None = None):
     X = X.contiguous()
     n, p = X.shape
     ld = (n + 15) // 16 * 16 if ld is None else int(ld)
-    codes = torch.zeros((p, ld), dtype=torch.uint8, device=X.device)
+    codes = torch.empty((p, ld), dtype=torch.uint8, device=X.device)
+    if ld > n:
+        codes[:, n:].zero_()  # the padding; the encoder writes the rest
     dims = torch.empty(p, dtype=torch.uint8, device=X.device)
     L = _lib.lib()
     ws = torch.empty(int(L.gcsl_encode_workspace_bytes(p)), dtype=torch.uint8, device=X.device)
