@@ -1015,7 +1015,29 @@ namespace host {
 // (p = 20, n = 1000: 63 splits of one step against 8 of eight).
 constexpr int OZ_MIN_STEPS = 8;
 
-// splits: K splits of the tile grid; 0 chooses one wave over num_sms SMs
+// K splits of a tile grid that fills more than half of a wave.  Whole tiles leave the last
+// wave partly empty (272 tiles of p = 1999 on 152 SMs: 1.79 waves that take 2); s splits make
+// it one s-th as long.  A split costs partial sums to write and read again and a prologue and
+// drain a block, 3 % of a split of OZ_LONG_SPLIT steps; counted as 1 % each, so that a split
+// more has to earn it.  The choice among the s that n allows grows with n only, and with it
+// the workspace.  p = 1999, n = 49999: five splits, product 3520 -> 3260 us.
+constexpr int OZ_LONG_SPLIT = 400, OZ_WAVE_SPLITS = 8;
+static int wave_splits(int tiles, long long steps, int num_sms) {
+    int best = 1;
+    double cost = 0.0;
+    for (int s = 1; s <= OZ_WAVE_SPLITS && (s == 1 || steps / s >= OZ_LONG_SPLIT); ++s) {
+        const long long blocks = (long long)tiles * s;
+        const double c = (double)((blocks + num_sms - 1) / num_sms) * num_sms / (double)blocks + 0.01 * s;
+        if (s == 1 || c < cost) {
+            cost = c;
+            best = s;
+        }
+    }
+    return best;
+}
+
+// splits: K splits of the tile grid; 0 chooses one wave over num_sms SMs, or a number that
+// fills the last of several
 static OzDims oz_dims(long long n, int p, int num_sms, int splits_req = 0) {
     OzDims D;
     D.p = p;
@@ -1027,7 +1049,7 @@ static OzDims oz_dims(long long n, int p, int num_sms, int splits_req = 0) {
     for (int i = 0; i < n_tiles_i; ++i) tiles += D.n_tiles_j - 2 * i;
     const long long steps = D.n_pad / 16;
     int splits = splits_req > 0 ? splits_req : num_sms / tiles;  // one wave: tiles x splits <= SMs
-    if (splits < 1) splits = 1;
+    if (splits_req <= 0 && splits < 2) splits = wave_splits(tiles, steps, num_sms);
     if (splits_req <= 0 && splits > (steps + OZ_MIN_STEPS - 1) / OZ_MIN_STEPS)
         splits = (int)((steps + OZ_MIN_STEPS - 1) / OZ_MIN_STEPS);
     if (splits > steps) splits = (int)steps;
@@ -1296,11 +1318,29 @@ static size_t batch_header_bytes(int count) {
     return batch_maps_offset(count) + ((size_t)count * 4 * sizeof(CUtensorMap) + 255) / 256 * 256;
 }
 
+// K steps of a batch's longest splits: a quarter of an SM's share of all tiles' steps, so that
+// the last blocks to start are short against the whole (one block per tile: the longest tile of
+// a small batch was twice an SM's share), within bounds that keep a block's fixed cost (about
+// ten steps) small and let the few problems of an exact rerun spread over the SMs.
+// 24 problems: product 642 -> 395 us; the exact rerun of a split batch of 256: 707 -> 474 us.
+static long long batch_split_steps(const long long *n, const int *p, int count) {
+    long long total = 0;
+    for (int k = 0; k < count; ++k) {
+        const OzDims D = oz_dims(n[k], p[k], 1, 1);
+        total += (long long)oz_tiles(D) * (D.n_pad / 16);
+    }
+    return std::min(512ll, std::max(128ll, total / (4 * 152)));
+}
+static int batch_splits(long long n, long long split_steps) {
+    return (int)std::max(1ll, ((n + 15) / 16 + split_steps - 1) / split_steps);
+}
+
 size_t corr_tc_batch_workspace_bytes(const long long *n, const int *p, int count) {
     size_t total = batch_header_bytes(count);
+    const long long split_steps = batch_split_steps(n, p, count);
     for (int k = 0; k < count; ++k) {
         OzJob J;
-        total += oz_job(J, nullptr, nullptr, n[k], p[k], p[k], 1, 1);
+        total += oz_job(J, nullptr, nullptr, n[k], p[k], p[k], 1, batch_splits(n[k], split_steps));
     }
     return total;
 }
@@ -1313,9 +1353,10 @@ cudaError_t corr_tc_batch_prepare(const void *const *X, const long long *n, cons
     std::vector<long long> off((size_t)OZ_NSTAGES * (count + 1), 0);
     char *base = static_cast<char *>(ws);
     size_t cur = batch_header_bytes(count);
+    const long long split_steps = batch_split_steps(n, p, count);
     for (int k = 0; k < count; ++k) {
         OzJob &J = jobs[(size_t)k];
-        cur += oz_job(J, base + cur, X[k], n[k], p[k], ldx[k], 1, 1);
+        cur += oz_job(J, base + cur, X[k], n[k], p[k], ldx[k], 1, batch_splits(n[k], split_steps));
         J.C = C[k];
         J.C32 = C32 ? C32[k] : nullptr;
         J.index = k;

@@ -49,7 +49,7 @@ def test_extreme_columns(cuda, n, p, dtype):
 
 
 def test_batch_equals_single(cuda):
-    """Batched jobs (one K range per tile) and single ones (K splits) give the same bits."""
+    """Batched jobs and single ones, whose K splits differ, give the same bits."""
     from gpucsl_gb300 import engine
     from gpucsl_gb300.batch import GaussianBatch
 
