@@ -88,6 +88,20 @@ __device__ __forceinline__ float f64_to_f32_rn(double v) {
     return __uint_as_float(fb);
 }
 
+// Tile `tile` of the upper triangle (bi <= bj) of an nb x nb grid, counted row by row: the
+// root of the quadratic in FP32, then at most a step or two.  (Counting the rows off took 157
+// dependent steps a block at p = 5000.)
+__device__ __forceinline__ void upper_tile(int tile, int nb, int &bi, int &bj) {
+    const float s = 2.0f * (float)nb + 1.0f;
+    int b = (int)(0.5f * (s - sqrtf(fmaxf(s * s - 8.0f * (float)tile, 0.0f))));
+    b = min(max(b, 0), nb - 1);
+    auto first = [nb](int r) { return r * nb - r * (r - 1) / 2; };  // first tile of row r
+    while (first(b) > tile) --b;
+    while (first(b + 1) <= tile) ++b;
+    bi = b;
+    bj = b + (tile - first(b));
+}
+
 // Programmatic dependent launch.  A kernel launched by launch_pdl may begin while the
 // kernel before it in the stream is still running: it must call pdl_wait() before it
 // reads anything that kernel wrote (a no-op when launched normally), and pdl_trigger()

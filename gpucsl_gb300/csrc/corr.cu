@@ -46,12 +46,8 @@ __global__ void __launch_bounds__(256) cov_tile_kernel(const T *__restrict__ X, 
                                                        double *__restrict__ C) {
     // map linear block id to an upper-triangle tile (bi <= bj)
     const int nb = (p + CT - 1) / CT;
-    int rem = blockIdx.x, bi = 0;
-    while (rem >= nb - bi) {
-        rem -= nb - bi;
-        ++bi;
-    }
-    const int bj = bi + rem;
+    int bi, bj;
+    upper_tile((int)blockIdx.x, nb, bi, bj);
     const int i0 = bi * CT, j0 = bj * CT;
 
     __shared__ double As[CK][CT];

@@ -934,12 +934,8 @@ __global__ void __launch_bounds__(256, 3) ozaki_finish_kernel(Src src) {
     if (src.skip(J.index)) return;
     const int p = J.p;
     const int nb = (p + 31) / 32;
-    int rem = (int)lb, bi = 0;
-    while (rem >= nb - bi) {
-        rem -= nb - bi;
-        ++bi;
-    }
-    const int bj = bi + rem;
+    int bi, bj;
+    upper_tile((int)lb, nb, bi, bj);
     const double scale = 1.0 / (double)(J.n - 1);
     const bool failed = *J.err != 0;  // a tensor-core wait timed out: poison the output
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
