@@ -294,12 +294,8 @@ __global__ void batch_level0_kernel(const BInst *__restrict__ inst, const long l
         const double eps = *I.c_err * 1.001 + 1e-15;
         const double t0 = sqrt(I.t2[0]);
         const int nb = (I.p + 31) / 32;
-        int rem = (int)lb, bi = 0;
-        while (rem >= nb - bi) {
-            rem -= nb - bi;
-            ++bi;
-        }
-        const int bj = bi + rem;
+        int bi, bj;
+        upper_tile((int)lb, nb, bi, bj);
         bool unsure = false;
         for (int r = threadIdx.x >> 5; r < 32; r += blockDim.x >> 5) {
             const int i = bi * 32 + r, j = bj * 32 + (threadIdx.x & 31);
@@ -372,6 +368,14 @@ __global__ void batch_edge_offsets_kernel(const long long *__restrict__ edges, i
 // FP32 tests need few registers, and the 24 resident warps hide more of the gathers'
 // latency than the 16 that the register count of their rare FP64 re-test path allowed
 // (a few spilled values of that path stay in L1).  Higher levels keep their registers.
+//
+// A group of lanes takes runs of consecutive edges (up to BATCH_RUN, fewer when there are not
+// four runs for every group): it finds the instance and row of the first by bisection and
+// steps on from there, adds a run's counts to the instance's with one atomic each, and its
+// neighbours' rows of C stay in L1.  An edge at a time, the two bisections (16 dependent loads)
+// and the atomics of all warps on the counters of one instance bounded the level.
+// 256 problems, all their levels: 2985 -> 2692 us (level 1: 1741 -> 1481).
+constexpr int BATCH_RUN = 8;
 template <int L, int G, bool SPLIT>
 __global__ void __launch_bounds__(256, (L <= 2 ? 3 : 1)) batch_level_kernel(const BInst *__restrict__ inst,
                                                          const long long *__restrict__ edge_off, int count,
@@ -382,48 +386,90 @@ __global__ void __launch_bounds__(256, (L <= 2 ? 3 : 1)) batch_level_kernel(cons
     const unsigned gbits = (G == 32) ? 0xffffffffu : ((1u << G) - 1u);
     const long long n_edges = edge_off[count];
     const long long warps = ((long long)gridDim.x * blockDim.x) >> 5;
+    // per group, in shared memory for the registers: tests made, tests of all keys, removals
+    __shared__ unsigned long long s_sums[256 / G][3];
+    unsigned long long *sums = s_sums[threadIdx.x / G];
+    if (gl == 0) sums[0] = sums[1] = sums[2] = 0;
+    const long long spare = n_edges / (warps * GPW * 4);
+    const int run = spare < 1 ? 1 : (spare < BATCH_RUN ? (int)spare : BATCH_RUN);
     const double inf = __longlong_as_double(0x7ff0000000000000ll);
-    for (long long e0 = (((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * GPW; e0 < n_edges;
-         e0 += warps * GPW) {
-        const long long e = e0 + gw;
-        const bool has = e < n_edges;
-        long long le = 0;
-        const int k = has ? inst_of(edge_off, count, e, le) : 0;
-        const BInst &I = inst[k];
-        EdgeJob J;
-        J.T = 0;
-        if (has && !load_edge<L>(I.adj, I.up, I.prefix, I.p, le, L, J)) {
-            if (gl == 0) set_status(I.st, GCSL_ERR_UNSUPPORTED);
+    for (long long w0 = (((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * (GPW * run); w0 < n_edges;
+         w0 += warps * (GPW * run)) {
+        // the edge's instance, its number there and the instance's count; its row, and the
+        // first edges of that and of the next row (an instance has fewer than 2^31 edges)
+        int k = 0, le = -1, n_le = 0, row = 0, r0 = 0, r1 = 0;
+        // adds the counts of the run's edges in instance k to the instance's
+        auto flush = [&]() {
+            if (gl == 0 && sums[1] != 0) {
+                DevState *st = inst[k].st;
+                atomicAdd(&st->tests[L], sums[0]);
+                atomicAdd(&st->tests_full[L], sums[1]);
+                if (sums[2]) atomicAdd(&st->removed[L], sums[2]);
+                sums[0] = sums[1] = sums[2] = 0;
+            }
+        };
+        for (int q = 0; q < run; ++q) {
+            const long long e = w0 + gw * run + q;
+            const bool has = e < n_edges;
+            ++le;
+            if (has && le >= n_le) {
+                flush();
+                k = upper_row(edge_off, count, e);
+                le = (int)(e - edge_off[k]);
+                n_le = (int)(edge_off[k + 1] - edge_off[k]);
+                const long long *prefix = inst[k].prefix;
+                row = upper_row(prefix, inst[k].p, le);
+                r0 = (int)prefix[row];
+                r1 = (int)prefix[row + 1];
+            }
+            const BInst &I = inst[k];
+            EdgeJob J;
             J.T = 0;
+            if (has) {
+                while (le >= r1) {
+                    ++row;
+                    r0 = r1;
+                    r1 = (int)I.prefix[row + 1];
+                }
+                const int *ra = I.adj + (size_t)row * I.p;
+                const int deg = ra[0], hi = ra[1 + (deg - I.up[row]) + le - r0];
+                edge_job_from<L>(row, hi, deg, I.adj[(size_t)hi * I.p], L, J);
+                if (J.R0 >= GCSL_RANK_LIMIT || J.R1 >= GCSL_RANK_LIMIT) {
+                    if (gl == 0) set_status(I.st, GCSL_ERR_UNSUPPORTED);
+                    J.T = 0;
+                }
+            }
+            double r2min = inf, zmin_exact = inf;
+            bool removed = false;
+            unsigned long long n_tests = 0, retests = 0;
+            if constexpr (SPLIT) {
+                // the rerun has the exact C: no bound
+                const double eps = (has && !rerun && I.c_err != nullptr) ? *I.c_err : -1.0;
+                // eps widened by 0.1 % in FP32, rounded up (no FP64 instruction per edge)
+                const float eps32 = __fmul_ru(f64_nonneg_to_f32_ru(eps), 1.001f);
+                walk_edge<L, G>(J, has, I.adj, I.p, gl, gshift, gbits,
+                                SplitTest<L>{I.C, I.C32, I.p, I.tau[L], I.t2[L], I.t2lo[L], I.t2hi[L], &retests, eps,
+                                             eps32, I.flag},
+                                I.G, nullptr, BATCH_MAX_LEVEL, I.rec, I.rec_cap, I.st, r2min, zmin_exact, removed,
+                                n_tests);
+            } else {
+                walk_edge<L, G>(J, has, I.adj, I.p, gl, gshift, gbits, F64Test<L>{I.C, I.p, I.tau[L], I.t2[L]}, I.G,
+                                nullptr, BATCH_MAX_LEVEL, I.rec, I.rec_cap, I.st, r2min, zmin_exact, removed, n_tests);
+            }
+            if (SPLIT && retests) atomicAdd(&I.st->retests, retests);
+            if (has && gl == 0 && J.T > 0) {
+                const size_t ix = (size_t)J.lo * I.p + J.hi;
+                // both non-negative for a pair alive at this level (integer compares, as in walk_edge)
+                if (__double_as_longlong(zmin_exact) < __double_as_longlong(inf))
+                    I.zmin[ix] = min_nonneg(I.zmin[ix], zmin_exact);
+                if (__double_as_longlong(r2min) < __double_as_longlong(inf))
+                    I.r2min[ix] = min_nonneg(I.r2min[ix], r2min);
+                sums[0] += n_tests;
+                sums[1] += (unsigned long long)J.T;
+                sums[2] += removed;
+            }
         }
-        double r2min = inf, zmin_exact = inf;
-        bool removed = false;
-        unsigned long long n_tests = 0, retests = 0;
-        if constexpr (SPLIT) {
-            // the rerun has the exact C: no bound
-            const double eps = (has && !rerun && I.c_err != nullptr) ? *I.c_err : -1.0;
-            // eps widened by 0.1 % in FP32, rounded up (no FP64 instruction per edge)
-            const float eps32 = __fmul_ru(f64_nonneg_to_f32_ru(eps), 1.001f);
-            walk_edge<L, G>(J, has, I.adj, I.p, gl, gshift, gbits,
-                            SplitTest<L>{I.C, I.C32, I.p, I.tau[L], I.t2[L], I.t2lo[L], I.t2hi[L], &retests, eps, eps32,
-                                         I.flag},
-                            I.G, nullptr, BATCH_MAX_LEVEL, I.rec, I.rec_cap, I.st, r2min, zmin_exact, removed,
-                            n_tests);
-        } else {
-            walk_edge<L, G>(J, has, I.adj, I.p, gl, gshift, gbits, F64Test<L>{I.C, I.p, I.tau[L], I.t2[L]}, I.G,
-                            nullptr, BATCH_MAX_LEVEL, I.rec, I.rec_cap, I.st, r2min, zmin_exact, removed, n_tests);
-        }
-        if (SPLIT && retests) atomicAdd(&I.st->retests, retests);
-        if (has && gl == 0 && J.T > 0) {
-            const size_t ix = (size_t)J.lo * I.p + J.hi;
-            // both non-negative for a pair alive at this level (integer compares, as in walk_edge)
-            if (__double_as_longlong(zmin_exact) < __double_as_longlong(inf))
-                I.zmin[ix] = min_nonneg(I.zmin[ix], zmin_exact);
-            if (__double_as_longlong(r2min) < __double_as_longlong(inf)) I.r2min[ix] = min_nonneg(I.r2min[ix], r2min);
-            atomicAdd(&I.st->tests[L], n_tests);
-            atomicAdd(&I.st->tests_full[L], (unsigned long long)J.T);
-            if (removed) atomicAdd(&I.st->removed[L], 1ull);
-        }
+        flush();
     }
 }
 
