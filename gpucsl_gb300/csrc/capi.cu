@@ -616,8 +616,6 @@ int gcsl::host::gauss_skeleton_run(const double *C, int p, long long n_obs, cons
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const int sms = device_sms();
     if (cudaMemsetAsync(w.st, 0, sizeof(DevState), s) != cudaSuccess) return GCSL_ERR_DEVICE;
-    // r2min starts at 0x7f7f... = 1.4e306, above every rho^2 < 1 the levels can store
-    if (cudaMemsetAsync(w.r2min, 0x7f, sizeof(double) * (size_t)p * p, s) != cudaSuccess) return GCSL_ERR_DEVICE;
     LevelTimer *lt = stats && !allocation_free ? level_timer() : nullptr;
     int n_timed = 0;  // events recorded: ev[0 .. n_timed]
     if (lt) cudaEventRecord(lt->ev[0], s);

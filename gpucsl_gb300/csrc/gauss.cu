@@ -296,7 +296,9 @@ __global__ void __launch_bounds__(256) pmax_kept_kernel(const int *__restrict__ 
 // Every other entry: pairs removed at level 0 (marker zmin = -1) get z* = Z(r) with
 // r = C[i*p + j] (gaussian_ci.cu:36-37), the lower triangle and diagonal -1.  Launched on
 // a second stream right after level 0; the later levels never touch these entries, so it
-// runs concurrently with them.  FP64 pipe: 785 us at p = 5000 with the two-step evaluation.
+// runs concurrently with them.  FP64 pipe: 785 us at p = 5000 with the two-step evaluation,
+// 295 with twelve FP64 operations a pair and one entry in flight, 250 with eight and four.
+constexpr unsigned PMAX_SPAN = 1024;  // entries of a block's step: four a thread
 __global__ void __launch_bounds__(256) pmax_level0_kernel(const double *__restrict__ C, const double *__restrict__ zmin,
                                                           int p, double sqrt_nm3, const double *__restrict__ sftab,
                                                           RTab R, double *__restrict__ pmax) {
@@ -304,11 +306,8 @@ __global__ void __launch_bounds__(256) pmax_level0_kernel(const double *__restri
     pmax_tables_load(S, sftab, R);
     __syncthreads();
     const unsigned total = (unsigned)p * (unsigned)p;  // p <= 46340: fits in 31 bits
-    for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k < total; k += gridDim.x * blockDim.x) {
-        const int i = (int)(k / (unsigned)p), j = (int)(k - (unsigned)i * (unsigned)p);
-        if (i >= j) pmax[k] = -1.0;
-        else if (zmin[k] < 0.0) pmax[k] = pmax_removed(S, R, sqrt_nm3, C[k]);
-    }
+    for (unsigned k = blockIdx.x * PMAX_SPAN; k < total; k += gridDim.x * PMAX_SPAN)
+        pmax_level0_span(S, R, C, zmin, (unsigned)p, sqrt_nm3, pmax, k, min(total, k + PMAX_SPAN));
 }
 
 // Unit kernel: all positions of ranks [0, count) (one thread per rank).
@@ -507,7 +506,7 @@ size_t pmax_table_doubles() { return (size_t)RT_CENTRES * RT_TERMS; }
 cudaError_t launch_pmax_level0(const double *C, const double *zmin, int p, long long n_obs, const double *sftab,
                                const double *rt, double tau, double *pmax, int num_sms, cudaStream_t s) {
     const long long total = (long long)p * p;
-    const long long want = (total + 255) / 256;
+    const long long want = (total + PMAX_SPAN - 1) / PMAX_SPAN;
     const int blocks = (int)(want < (long long)num_sms * 4 ? want : (long long)num_sms * 4);
     const RTab R = rt_params(n_obs, tau, (long long)p * (p - 1) / 2, rt);
     pmax_level0_kernel<<<blocks > 0 ? blocks : 1, 256, 0, s>>>(C, zmin, p, sqrt((double)(n_obs - 3)), sftab, R, pmax);

@@ -265,22 +265,13 @@ __device__ __forceinline__ int inst_of(const long long *__restrict__ off, int co
 // A kernel of the exact re-solve (rerun) skips every instance whose flag is not set.
 __device__ __forceinline__ bool skip_inst(const BInst &I, bool rerun) { return rerun && *(volatile int *)I.flag == 0; }
 
-// Per p^2 chunk: r2min = 1.4e306 (above every stored rho^2); chunk 0 also clears the
-// instance's DevState (and, on the first pass, its flag).
-__global__ void batch_init_kernel(const BInst *__restrict__ inst, const long long *__restrict__ off_p2, int count,
-                                  bool rerun) {
-    long long lb;
-    const BInst &I = inst[inst_of(off_p2, count, blockIdx.x, lb)];
+// Clears an instance's DevState (and, on the first pass, its flag); block = instance.
+__global__ void batch_init_kernel(const BInst *__restrict__ inst, bool rerun) {
+    const BInst &I = inst[blockIdx.x];
     if (skip_inst(I, rerun)) return;
-    if (lb == 0 && !rerun && threadIdx.x == 0) *I.flag = 0;
-    const long long total = (long long)I.p * I.p;
-    const long long k0 = lb * BATCH_P2_CHUNK, k1 = min(total, k0 + BATCH_P2_CHUNK);
-    const double big = __longlong_as_double(0x7f7f7f7f7f7f7f7fll);
-    for (long long k = k0 + threadIdx.x; k < k1; k += blockDim.x) I.r2min[k] = big;
-    if (lb == 0) {
-        unsigned *w = reinterpret_cast<unsigned *>(I.st);
-        for (int k = threadIdx.x; k < (int)(sizeof(DevState) / sizeof(unsigned)); k += blockDim.x) w[k] = 0u;
-    }
+    if (!rerun && threadIdx.x == 0) *I.flag = 0;
+    unsigned *w = reinterpret_cast<unsigned *>(I.st);
+    for (int k = threadIdx.x; k < (int)(sizeof(DevState) / sizeof(unsigned)); k += blockDim.x) w[k] = 0u;
 }
 
 // Level 0.  On an approximate C (first pass, c_err set) a pair whose |r| lies within the
@@ -487,11 +478,7 @@ __global__ void __launch_bounds__(256) batch_pmax_removed_kernel(const BInst *__
     const unsigned p = (unsigned)I.p;
     const unsigned total = p * p;
     const unsigned k0 = (unsigned)lb * BATCH_P2_CHUNK, k1 = min(total, k0 + (unsigned)BATCH_P2_CHUNK);
-    for (unsigned k = k0 + threadIdx.x; k < k1; k += blockDim.x) {
-        const unsigned i = k / p, j = k - i * p;
-        if (i >= j) I.pmax[k] = -1.0;
-        else if (I.zmin[k] < 0.0) I.pmax[k] = pmax_removed(S, R, I.sqrt_nm3, I.C[k]);
-    }
+    pmax_level0_span(S, R, I.C, I.zmin, p, I.sqrt_nm3, I.pmax, k0, k1);
 }
 
 // pmax of the pairs kept at level 0, BATCH_KEPT_BLOCKS blocks per instance (one block took
@@ -821,7 +808,7 @@ int gauss_batch_step(const long long *plan, int first, int last, bool finish, bo
     double *sftab = reinterpret_cast<double *>(base + Ly.sftab), *rt = reinterpret_cast<double *>(base + Ly.rt);
 
     if (first == 0) {
-        batch_init_kernel<<<(unsigned)plan[PW_P2], 256, 0, s>>>(inst, op2, count, rerun);
+        batch_init_kernel<<<(unsigned)count, 256, 0, s>>>(inst, rerun);
         batch_level0_kernel<<<(unsigned)plan[PW_TILES], 256, 0, s>>>(inst, ot, count, rerun);
         note_launch(2);
     }

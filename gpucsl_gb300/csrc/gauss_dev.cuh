@@ -13,8 +13,8 @@ namespace gcsl {
 // 32 x 32 tiles of the upper triangle (tile row bi <= tile column bj): for i < j,
 // Z = |0.5 log|(1+r)/(1-r)||, r = C[i*p + j]; remove iff Z < tau0, decided as
 // r^2 < tanh(tau0)^2 away from the knife edge.  Kept pairs store r^2 in r2min (zmin =
-// +inf; the exact Z only where the reference formula decided) and append i * p + j to
-// `kept`; removed pairs store the marker zmin = -1: their z* is final and their pmax is
+// +inf; where the reference formula decided, the exact Z and an r2min above every rho^2) and
+// append i * p + j to `kept`; removed pairs store the marker zmin = -1: their z* is final and their pmax is
 // computed from C by pmax_level0_kernel, concurrently with the later levels.
 // The mirrored skeleton entries are written through a shared-memory transpose so both
 // triangles are stored row-contiguously; zero diagonal.
@@ -71,7 +71,8 @@ __device__ __forceinline__ void level0_tile(const double *__restrict__ C, int p,
                 z = fabs(0.5 * log(fabs((1.0 + c) / (1.0 - c))));
                 rem0 = z < tau0;
                 if (rem0) z = -1.0;
-                else if (isnan(z)) z = __longlong_as_double(0x7ff0000000000000ll);
+                else r2min[(size_t)i * p + j] = __longlong_as_double(0x7f7f7f7f7f7f7f7fll);  // 1.4e306
+                if (isnan(z)) z = __longlong_as_double(0x7ff0000000000000ll);
             }
             g = rem0 ? 0 : 1;
             zmin[(size_t)i * p + j] = z;
@@ -972,20 +973,22 @@ __device__ __forceinline__ double fisher_z(double r) {
 
 // pmax of a pair straight from |rho|: f(r) = erfc(c atanh r), c = sqrt((n - 3) / 2), by Taylor
 // expansions about RT_CENTRES equidistant centres r = m w on [0, rmax].  Evaluating Z and
-// erfc one after the other takes about 36 FP64 operations a pair, this 10 -- on a pipe of
-// 1/64 of the FP32 rate they are the time of the pmax kernels.  rmax covers the pairs that a
+// erfc one after the other takes about 36 FP64 operations a pair, this 8 (the centre is found
+// in FP32, comparisons are on the bits) -- on a pipe of 1/64 of the FP32 rate they are the time
+// of the pmax kernels.  rmax covers the pairs that a
 // test removed (|rho| below tanh of the largest threshold); the others, |rho| >= 1 and exact Z
 // minima take the evaluation above.  With c atanh(rmax) <= 3 and rmax <= 1/2 (rt_params) eight
 // terms leave a truncation below 6e-17 of the value; against 40 digits the error is below
 // 3e-15 relative over n = 30 .. 50000 and alpha = 2.5e-5 .. 0.05, smaller than that of the
 // two-step evaluation everywhere (it does not round the argument of erfc).
 constexpr int RT_CENTRES = 256, RT_TERMS = 8;
-constexpr int RT_STRIDE = RT_TERMS + 1;  // in shared memory: lanes at different centres meet different banks
+constexpr int RT_STRIDE = RT_TERMS + 1;  // in shared memory, with the centre: an odd stride spreads the banks
 
 struct RTab {
     const double *a;          // RT_CENTRES x RT_TERMS coefficients in global memory, or null: not used
-    double w, inv_w, rmax, rmax2;
+    double w, rmax, rmax2;
     double c;
+    float inv_w;
 };
 
 // The table's parameters for n observations and largest threshold tau; a stays null where
@@ -997,7 +1000,7 @@ __host__ inline RTab rt_params(long long n_obs, double tau, long long pairs, con
     R.rmax = std::tanh(tau) * (1.0 + 1e-6);
     R.rmax2 = R.rmax * R.rmax * (1.0 - 1e-12);
     R.w = R.rmax / (RT_CENTRES - 1);
-    R.inv_w = R.w > 0.0 ? 1.0 / R.w : 0.0;
+    R.inv_w = R.w > 0.0 ? (float)(1.0 / R.w) : 0.0f;
     const bool ok = pairs >= 8192 && tau > 0.0 && R.rmax <= 0.5 && R.c * std::atanh(R.rmax) <= 3.0;  // false for NaN
     if (ok) R.a = a;
     return R;
@@ -1036,20 +1039,22 @@ __device__ __forceinline__ void rt_build(const RTab &R, int m, double *__restric
     }
 }
 
-// The table into a block's shared memory (RT_CENTRES * RT_STRIDE doubles).
-__device__ __forceinline__ void rt_load(double *__restrict__ sm, const double *__restrict__ a) {
+// The table and its centres into a block's shared memory (RT_CENTRES * RT_STRIDE doubles).
+__device__ __forceinline__ void rt_load(double *__restrict__ sm, const RTab &R) {
     for (int k = threadIdx.x; k < RT_CENTRES * RT_TERMS; k += blockDim.x)
-        sm[(k / RT_TERMS) * RT_STRIDE + k % RT_TERMS] = __ldg(a + k);
+        sm[(k / RT_TERMS) * RT_STRIDE + k % RT_TERMS] = __ldg(R.a + k);
+    for (int m = threadIdx.x; m < RT_CENTRES; m += blockDim.x) sm[m * RT_STRIDE + RT_TERMS] = m * R.w;
 }
 
-// f(r) for 0 <= r < rmax: the nearest centre by adding 1.5 * 2^52 (the sum's low bits are the
-// rounded quotient), then Horner.
+// f(r) for 0 <= r < rmax: the nearest centre (in FP32 from the leading bits of r, off by less
+// than 1e-4 of a step at the middle between two; adding 1.5 * 2^23 rounds), then Horner.
 __device__ __forceinline__ double rt_eval(const RTab &R, const double *__restrict__ sm, double r) {
-    constexpr double magic = 6755399441055744.0;
-    const double v = fma(r, R.inv_w, magic);
-    const unsigned m = min((unsigned)__double_as_longlong(v), (unsigned)(RT_CENTRES - 1));
-    const double t = fma(-(v - magic), R.w, r);
+    const unsigned hi = (unsigned)__double2hiint(r);
+    const unsigned f32 = hi < 0x38100000u ? 0u : __funnelshift_l((unsigned)__double2loint(r), hi - 0x38000000u, 3);
+    const unsigned v = __float_as_uint(fmaf(__uint_as_float(f32), R.inv_w, 12582912.0f));
+    const unsigned m = min(v & 0xfffu, (unsigned)(RT_CENTRES - 1));
     const double *a = sm + m * RT_STRIDE;
+    const double t = r - a[RT_TERMS];
     double f = a[RT_TERMS - 1];
 #pragma unroll
     for (int k = RT_TERMS - 2; k >= 0; --k) f = fma(f, t, a[k]);
@@ -1063,14 +1068,42 @@ struct PmaxShared {
 };
 __device__ __forceinline__ void pmax_tables_load(PmaxShared &S, const double *__restrict__ sftab, const RTab &R) {
     sf_table_load(S.sf, sftab);
-    if (R.a != nullptr) rt_load(S.rt, R.a);
+    if (R.a != nullptr) rt_load(S.rt, R);
 }
 
 // pmax of a pair removed at level 0, from its correlation.
 __device__ __forceinline__ double pmax_removed(const PmaxShared &S, const RTab &R, double sqrt_nm3, double c) {
     const double r = fabs(c);
-    if (R.a != nullptr && r < R.rmax) return rt_eval(R, S.rt, r);
+    // (compared on the bits: NaN is above every number)
+    if (R.a != nullptr && __double_as_longlong(r) < __double_as_longlong(R.rmax)) return rt_eval(R, S.rt, r);
     return two_sf_tab(sqrt_nm3 * fisher_z(c), S.sf);
+}
+
+// Entries [k0, k1) of a p x p pmax matrix by one block: pairs removed at level 0 (marker
+// zmin = -1) get theirs from C, the lower triangle and diagonal -1, the others nothing.  Four
+// entries a thread in flight.
+__device__ __forceinline__ void pmax_level0_span(const PmaxShared &S, const RTab &R, const double *__restrict__ C,
+                                                 const double *__restrict__ zmin, unsigned p, double sqrt_nm3,
+                                                 double *__restrict__ pmax, unsigned k0, unsigned k1) {
+    for (unsigned b = k0 + threadIdx.x; b < k1; b += 4 * blockDim.x) {
+        double c[4];
+        int mark[4];  // negative: removed at level 0; 1: not of the upper triangle
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const unsigned k = b + q * blockDim.x, i = k / p, j = k - i * p;
+            c[q] = 0.0;
+            mark[q] = k < k1 && i >= j ? 1 : 0;
+            if (k < k1 && i < j) {
+                c[q] = C[k];
+                mark[q] = __double2hiint(zmin[k]) < 0 ? -1 : 0;
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            if (mark[q] == 0) continue;
+            pmax[b + q * blockDim.x] = mark[q] > 0 ? -1.0 : pmax_removed(S, R, sqrt_nm3, c[q]);
+        }
+    }
 }
 
 // pmax of the pairs kept at level 0, share b of nb blocks of 256 threads: z* = min(zmin, Z of
