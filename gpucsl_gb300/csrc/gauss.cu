@@ -87,8 +87,10 @@ __global__ void row_scan_kernel(const T *__restrict__ cnt, int p, long long *__r
 // count can be read before the wait.  Blocks beyond the bound leave before loading the
 // binomial rows (the upper levels keep a few hundred edges, and the grid is sized for
 // the thousands of level 1); block 0 always stays, it records the end of the loop.
+// Level 1 at three blocks an SM: 309 us at p = 5000, 321 at four (registers spilled), two by
+// the kernel's own count.
 template <int L, bool MIXED>
-__global__ void __launch_bounds__(256) gauss_level_reg_kernel(LevelCtx x) {
+__global__ void __launch_bounds__(256, L == 1 ? 3 : 1) gauss_level_reg_kernel(LevelCtx x) {
     __shared__ BinomRows sb;
     if (L >= 2 && blockIdx.x > 0 &&
         (long long)blockIdx.x * (blockDim.x >> 5) >= (long long)__ldcg(&x.st->edges[L - 1]))

@@ -381,32 +381,6 @@ __device__ __forceinline__ bool load_edge(const int *__restrict__ adj, const int
     return J.R0 < GCSL_RANK_LIMIT && J.R1 < GCSL_RANK_LIMIT;
 }
 
-// Edge e of the level from the explicit edge list (lo < hi) written by the edge scan.
-template <int KMAX>
-__device__ __forceinline__ bool load_edge_list(const int *__restrict__ adj, const int2 *__restrict__ elist, int p,
-                                               long long e, int L, EdgeJob &J, DevState *st = nullptr) {
-    const int2 ed = elist[e];
-    if (!dcheck(st, ed.x >= 0 && ed.x < ed.y && ed.y < p, GCSL_DCHECK_EDGE)) {  // no tests for this edge
-        J.lo = 0;
-        J.hi = p > 1 ? 1 : 0;
-        J.deg_lo = J.deg_hi = 0;
-        J.R0 = J.R1 = J.T = J.Rmin = 0;
-        J.longer = 0;
-        return true;
-    }
-    J.lo = ed.x;
-    J.hi = ed.y;
-    J.deg_lo = adj[(size_t)ed.x * p];
-    J.deg_hi = adj[(size_t)ed.y * p];
-    const int K0 = J.deg_lo - 1, K1 = J.deg_hi - 1;
-    J.R0 = (K0 >= L) ? binom_fast<KMAX>(K0, L) : 0;
-    J.R1 = (K1 >= L) ? binom_fast<KMAX>(K1, L) : 0;
-    J.T = J.R0 + J.R1;
-    J.Rmin = J.R0 < J.R1 ? J.R0 : J.R1;
-    J.longer = J.R0 > J.R1 ? 0 : 1;
-    return J.R0 < GCSL_RANK_LIMIT && J.R1 < GCSL_RANK_LIMIT;
-}
-
 // The job of edge (lo, hi) from degrees already known (the unit kernel takes them from the
 // chunk record instead of reloading the adjacency rows' counts).
 template <int KMAX>
@@ -705,6 +679,56 @@ struct F64Test {
     }
 };
 
+// Candidate kernel body: the FP64 test of queued entry e, folded into the pair's minima.
+template <int L>
+__device__ __forceinline__ void eval_candidate(const double *__restrict__ C, int p, const int *e, double tau,
+                                               double t2, double *zmin, double *r2min,
+                                               const long long *__restrict__ chunk_first = nullptr) {
+    // a key of a chunked edge behind the edge's canonical remover does not count
+    if (e[3] >= 0 && chunk_first != nullptr && (long long)e[4] > chunk_first[e[3]]) return;
+    int S[L];
+#pragma unroll
+    for (int c = 0; c < L; ++c) S[c] = e[CAND_HEADER + c];
+    const TestOut o = gauss_test_reg<L>(C, p, e[1], e[2], S, tau, t2);
+    const size_t ix = (size_t)e[0];
+    if (o.rho2 < __longlong_as_double(0x7ff0000000000000ll)) atomic_min_nonneg_f64(r2min + ix, o.rho2);
+    if (o.zexact < __longlong_as_double(0x7ff0000000000000ll)) atomic_min_nonneg_f64(zmin + ix, o.zexact);
+}
+
+// Candidates of one warp gathered in shared memory on their way to the queue: a reservation
+// for every step of every edge put all warps of the grid on one counter and each of them in
+// front of its answer.
+constexpr int CAND_STAGE = 64;  // entries: flushed when a step's 32 might not fit any more
+struct CandStage {
+    int *buf;
+    int n;  // entries (the same in every lane)
+    double *zmin, *r2min;
+};
+
+template <int L>
+__device__ __noinline__ void eval_candidate_call(const double *__restrict__ C, int p, const int *e, double tau, double t2,
+                                                 double *zmin, double *r2min) {
+    eval_candidate<L>(C, p, e, tau, t2, zmin, r2min);
+}
+
+// Whole warp.  Entries that the queue has no room for are evaluated here.
+template <int L, class Test>
+__device__ __forceinline__ void flush_candidates(const Test &test, const CandQueue &q, CandStage &g) {
+    constexpr int W = CAND_HEADER + L;
+    if (g.n == 0) return;
+    const int lane = threadIdx.x & 31, ints = W * g.n;
+    __syncwarp();
+    unsigned long long b0 = 0;
+    if (lane == 0) b0 = atomicAdd(q.count, (unsigned long long)ints);
+    b0 = __shfl_sync(GCSL_FULL_MASK, b0, 0);
+    const long long room = q.cap - (long long)b0, keep = room < 0 ? 0 : (room < ints ? room / W * W : ints);
+    for (int k = lane; k < (int)keep; k += 32) q.buf[b0 + k] = g.buf[k];
+    for (int t = (int)keep / W + lane; t < g.n; t += 32)
+        eval_candidate_call<L>(test.C, test.p, g.buf + W * t, test.tau, test.t2, g.zmin, g.r2min);
+    __syncwarp();
+    g.n = 0;
+}
+
 // One G-lane group walks edge J's merged key sequence G keys at a time: each lane tests
 // one key, the lowest removing lane is the canonical remover (its set is written back),
 // and the keys up to it fold into the group's minima of rho^2 (r2min) and of the exactly
@@ -734,7 +758,7 @@ __device__ __forceinline__ void walk_edge(const EdgeJob &J, bool has, const int 
                                           DevState *st, double &r2min, double &zmin_exact, bool &removed,
                                           unsigned long long &n_tests, const CandQueue *q = nullptr,
                                           const BinomRows *sb = nullptr, double r2_floor = 0.0,
-                                          WalkRange *rg = nullptr) {
+                                          WalkRange *rg = nullptr, CandStage *stage = nullptr) {
     const double inf = __longlong_as_double(0x7ff0000000000000ll);
     // r2_floor rounded up to FP32: a key whose FP32 interval starts above it cannot lower
     // z* (the rounding only admits a few more candidates), compared in FP32 per step
@@ -786,7 +810,22 @@ __device__ __forceinline__ void walk_edge(const EdgeJob &J, bool has, const int 
             const float hi = group_min_f<G>((fold && !o.exact) ? __fadd_ru(o.r32, o.e32) : __int_as_float(0x7f800000));
             bool cand = fold && !o.exact && lo32 <= hi && lo32 <= floor32;
             const unsigned cm = __ballot_sync(GCSL_FULL_MASK, cand);
-            if (cm) {
+            if (cm && stage != nullptr) {  // (32-lane groups)
+                constexpr int W = CAND_HEADER + L;
+                if (cand) {
+                    int *e = stage->buf + W * (stage->n + __popc(cm & ((1u << (threadIdx.x & 31)) - 1u)));
+                    e[0] = J.lo * p + J.hi;
+                    e[1] = vi;
+                    e[2] = vj;
+                    e[3] = -1;
+                    e[4] = (int)m;
+#pragma unroll
+                    for (int c = 0; c < L; ++c) e[CAND_HEADER + c] = S[c];
+                    cand = false;
+                }
+                stage->n += __popc(cm);
+                if (stage->n > CAND_STAGE - 32) flush_candidates<L>(test, *q, *stage);
+            } else if (cm) {
                 constexpr int W = CAND_HEADER + L;
                 unsigned long long b0 = 0;
                 const int leader = __ffs(cm) - 1;
@@ -889,22 +928,6 @@ __device__ __forceinline__ bool register_chunked(const EdgeJob &J, int gl, const
         for (long long k = ub + gl; k < ub + nu && k < ck.unit_cap; k += G) ck.unit_h[k] = -1;
     }
     return ok;
-}
-
-// Candidate kernel body: the FP64 test of queued entry e, folded into the pair's minima.
-template <int L>
-__device__ __forceinline__ void eval_candidate(const double *__restrict__ C, int p, const int *e, double tau,
-                                               double t2, double *zmin, double *r2min,
-                                               const long long *__restrict__ chunk_first = nullptr) {
-    // a key of a chunked edge behind the edge's canonical remover does not count
-    if (e[3] >= 0 && chunk_first != nullptr && (long long)e[4] > chunk_first[e[3]]) return;
-    int S[L];
-#pragma unroll
-    for (int c = 0; c < L; ++c) S[c] = e[CAND_HEADER + c];
-    const TestOut o = gauss_test_reg<L>(C, p, e[1], e[2], S, tau, t2);
-    const size_t ix = (size_t)e[0];
-    if (o.rho2 < __longlong_as_double(0x7ff0000000000000ll)) atomic_min_nonneg_f64(r2min + ix, o.rho2);
-    if (o.zexact < __longlong_as_double(0x7ff0000000000000ll)) atomic_min_nonneg_f64(zmin + ix, o.zexact);
 }
 
 // ------------------------------------------------------------------ p-values

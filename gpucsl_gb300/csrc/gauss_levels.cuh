@@ -46,12 +46,12 @@ template <int L, bool MIXED>
 __device__ __forceinline__ void walk_level_keys(const EdgeJob &J, bool has, int lane, const LevelCtx &x,
                                                 double &r2min, double &zmin_exact, bool &removed,
                                                 unsigned long long &n_tests, const BinomRows *sb, double floor,
-                                                WalkRange *rg) {
+                                                WalkRange *rg, CandStage *stage = nullptr) {
     if constexpr (MIXED) {
         walk_edge<L, 32>(J, has, x.adj, x.p, lane, 0u, 0xffffffffu,
                          MixedTest<L>{x.C, x.mix.C32, x.p, x.tau, x.t2, x.mix.t2lo, x.mix.t2hi}, x.G, x.sep_dense,
                          x.max_level, x.rec_pool, x.rec_cap, x.st, r2min, zmin_exact, removed, n_tests, &x.mix.q, sb,
-                         floor, rg);
+                         floor, rg, stage);
     } else {
         walk_edge<L, 32>(J, has, x.adj, x.p, lane, 0u, 0xffffffffu, F64Test<L>{x.C, x.p, x.tau, x.t2}, x.G,
                          x.sep_dense, x.max_level, x.rec_pool, x.rec_cap, x.st, r2min, zmin_exact, removed, n_tests,
@@ -81,10 +81,49 @@ __device__ __forceinline__ void level_edge_phase(const LevelCtx &x, const BinomR
     // completed before this kernel's wait returned.
     const bool hand_over = x.ck.heavy != nullptr && L >= 3 &&
                            8ull * __ldcg(&st->removed[L - 1]) < __ldcg(&st->edges[L - 1]);
+    // At level 1, whose warps take dozens of edges (the upper levels' take one or none), the next
+    // edge's degrees and floor and the one after's ends are loaded ahead; with the
+    // candidates' staging below, level 1 at p = 5000 went from 431 to 309 us, at p = 1999 from
+    // 133 to 99 us (more warps an SM gained nothing while every step reserved queue space).
+    constexpr bool AHEAD = L == 1;
+    auto ends = [&](long long e0) { return x.elist[work_order(e0, n_edges, x.order)]; };
+    auto in_range = [&](int2 ed) { return ed.x >= 0 && ed.x < ed.y && ed.y < p; };
+    int2 ed1 = make_int2(0, 0), ed2 = ed1;
+    int deg_lo1 = 0, deg_hi1 = 0;
+    double floor1 = 0.0;
+    auto ahead = [&]() {
+        if (GCSL_DEBUG_CHECKS && !in_range(ed1)) return;  // no tests for this edge
+        deg_lo1 = x.adj[(size_t)ed1.x * p];
+        deg_hi1 = x.adj[(size_t)ed1.y * p];
+        // the pair's exact rho^2 minimum from earlier levels (level 0 stored r^2)
+        if (MIXED) floor1 = x.r2min[(size_t)ed1.x * p + ed1.y];
+    };
+    if (AHEAD && w0 < n_edges) {
+        ed1 = ends(w0);
+        if (w0 + nw < n_edges) ed2 = ends(w0 + nw);
+        ahead();
+    }
+    // level 1 (edges walked whole) gathers its candidates
+    __shared__ int s_stage[MIXED && L == 1 ? 8 * CAND_STAGE * (CAND_HEADER + L) : 1];
+    CandStage stage{s_stage + (MIXED && L == 1 ? (threadIdx.x >> 5) * (CAND_STAGE * (CAND_HEADER + L)) : 0), 0, x.zmin,
+                    x.r2min};
     for (long long e0 = w0; e0 < n_edges; e0 += nw) {
-        const long long e = work_order(e0, n_edges, x.order);
+        if (!AHEAD) {
+            ed1 = ends(e0);
+            ahead();
+        }
+        const int2 ed = ed1;
+        const int deg_lo = deg_lo1, deg_hi = deg_hi1;
+        const double floor = floor1;
+        if (AHEAD && e0 + nw < n_edges) {
+            ed1 = ed2;
+            ahead();
+            if (e0 + 2 * nw < n_edges) ed2 = ends(e0 + 2 * nw);
+        }
+        if (!dcheck(st, in_range(ed), GCSL_DCHECK_EDGE)) continue;
         EdgeJob J;
-        if (!load_edge_list<L>(x.adj, x.elist, p, e, L, J, st)) {
+        edge_job_from<L>(ed.x, ed.y, deg_lo, deg_hi, L, J);
+        if (J.R0 >= GCSL_RANK_LIMIT || J.R1 >= GCSL_RANK_LIMIT) {
             if (lane == 0) set_status(st, GCSL_ERR_UNSUPPORTED);
             J.T = 0;
         }
@@ -92,15 +131,14 @@ __device__ __forceinline__ void level_edge_phase(const LevelCtx &x, const BinomR
         if (J.T == 0) continue;
         double r2min = inf, zmin_exact = inf;
         bool removed = false;
-        // the pair's exact rho^2 minimum from earlier levels (level 0 stored r^2)
-        const double floor = MIXED ? x.r2min[(size_t)J.lo * p + J.hi] : 0.0;
         if (hand_over && register_chunked<32>(J, lane, x.ck, st, L, inf, inf, floor, 0))
             continue;  // tests, minima and the removal come from the unit phase
         // an edge with more than one step of keys walks its first step here; without a
         // remover there, the unit phase walks the rest in parallel
         const bool chunk = x.ck.heavy != nullptr && J.T > CHUNK_MIN_KEYS;
         WalkRange rg{0, chunk ? 32ll : J.T, false, -1, J.T};
-        walk_level_keys<L, MIXED>(J, true, lane, x, r2min, zmin_exact, removed, n_tests, sb, floor, &rg);
+        walk_level_keys<L, MIXED>(J, true, lane, x, r2min, zmin_exact, removed, n_tests, sb, floor, &rg,
+                                  L == 1 ? &stage : nullptr);
         bool deferred = false;
         if (chunk && !removed) {
             deferred = register_chunked<32>(J, lane, x.ck, st, L, r2min, zmin_exact, floor);
@@ -119,6 +157,8 @@ __device__ __forceinline__ void level_edge_phase(const LevelCtx &x, const BinomR
             n_removed += removed;
         }
     }
+    if constexpr (MIXED && L == 1)
+        flush_candidates<L>(MixedTest<L>{x.C, x.mix.C32, x.p, x.tau, x.t2, x.mix.t2lo, x.mix.t2hi}, x.mix.q, stage);
     if (lane == 0) {
         if (n_tests) atomicAdd(&st->tests[L], n_tests);
         if (n_full) atomicAdd(&st->tests_full[L], n_full);
