@@ -334,7 +334,16 @@ __global__ void col_mean_exp_kernel(Src src) {
     const int j = (int)lb * blockDim.x + threadIdx.x;
     if (j >= p) return;
     double s = 0.0;
-    for (int c = 0; c < J.chunks; ++c) s += J.partial[(size_t)c * p + j];
+    const double *__restrict__ part = J.partial + j;
+    int c = 0;
+    for (; c + 16 <= J.chunks; c += 16) {  // sixteen loads in flight, added in order (batch of 24: 15 -> 10 us)
+        double v[16];
+#pragma unroll
+        for (int e = 0; e < 16; ++e) v[e] = part[(size_t)(c + e) * p];
+#pragma unroll
+        for (int e = 0; e < 16; ++e) s += v[e];
+    }
+    for (; c < J.chunks; ++c) s += part[(size_t)c * p];
     const double mu = s / (double)J.n;
     J.mean[j] = mu;
     const double dev = fmax(key_value(J.kmax[j]) - mu, mu - key_value(J.kmin[j]));

@@ -88,7 +88,7 @@ __global__ void row_scan_kernel(const T *__restrict__ cnt, int p, long long *__r
 // binomial rows (the upper levels keep a few hundred edges, and the grid is sized for
 // the thousands of level 1); block 0 always stays, it records the end of the loop.
 // Level 1 at three blocks an SM: 309 us at p = 5000, 321 at four (registers spilled), two by
-// the kernel's own count.
+// the kernel's own count; nine launched an SM, three whole waves of them, 291 us (eight: 306).
 template <int L, bool MIXED>
 __global__ void __launch_bounds__(256, L == 1 ? 3 : 1) gauss_level_reg_kernel(LevelCtx x) {
     __shared__ BinomRows sb;
@@ -397,12 +397,12 @@ cudaError_t launch_gauss_level(int L, const double *C, int p, const int *adj, co
                                const ChunkBufs &ck, cudaStream_t s) {
     // register-heavy upper levels run 128-thread blocks
     const int threads = L >= 4 ? 128 : 256;
-    const int blocks = num_sms * 8;
+    const int blocks = num_sms * (L == 1 ? 9 : 8);
     const bool mixed = C32 != nullptr && qbuf != nullptr;
     const LevelCtx x = level_ctx(L, C, p, adj, elist, tau, tau_valid, G, zmin, r2min, sep_dense, max_level, rec_pool,
                                  rec_cap, st, C32, qbuf, qcap, ck);
     // chunked edges: the unit kernel follows the level kernel (it returns at once when no
-    // edge was chunked).  Both kernels launch 8 blocks per SM whose warps stride over the
+    // edge was chunked).  Both kernels launch 8 blocks per SM (level 1: nine) whose warps stride over the
     // edges / units: more than one resident wave at every level's register count, so blocks
     // of later waves pick up the work of the slow ones (measured on p = 1000: 0.771 ms per
     // solve against 0.801 ms with one resident wave and 0.80 / 0.85 ms with 16 / 32 per SM)
