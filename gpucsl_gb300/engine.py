@@ -188,10 +188,12 @@ class GaussianSolver:
 
 
 class DiscreteSolver:
-    """Discrete (chi-squared) PC-stable skeleton on one device."""
+    """Discrete (chi-squared) PC-stable skeleton on one device.  codes and dims: device tensors
+    laid out like `data` ((p, ld) uint8, ld = n rounded up to 16) and `dims` to take over
+    instead of allocating them and copying in load()."""
 
     def __init__(self, p: int, n: int, max_level: int, max_dim: int, device=None, record_cap: int | None = None,
-                 debug: bool = False):
+                 debug: bool = False, codes=None, dims=None):
         torch = _torch()
         self.p, self.n, self.max_level, self.max_dim = int(p), int(n), int(max_level), int(max_dim)
         self.device = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
@@ -200,13 +202,22 @@ class DiscreteSolver:
         L = _lib.lib(self.debug)
         ws = int(L.gcsl_disc_workspace_bytes(self.p, self.n, self.max_level, self.max_dim))
         self.workspace = torch.empty(ws, dtype=torch.uint8, device=self.device)
-        self.data = torch.zeros((self.p, self.ld), dtype=torch.uint8, device=self.device)
-        self.dims = torch.empty(self.p, dtype=torch.uint8, device=self.device)
-        self.G = torch.empty((self.p, self.p), dtype=torch.int16, device=self.device)
-        self.pmax = torch.empty((self.p, self.p), dtype=torch.float64, device=self.device)
+        if codes is not None and (tuple(codes.shape) != (self.p, self.ld) or not codes.is_contiguous()
+                                  or codes.data_ptr() % 16):
+            raise ValueError("codes must be a contiguous (p, n rounded up to 16) tensor on a 16-byte boundary")
+        self.data = torch.zeros((self.p, self.ld), dtype=torch.uint8, device=self.device) if codes is None else codes
+        self.dims = torch.empty(self.p, dtype=torch.uint8, device=self.device) if dims is None else dims
         if record_cap is None:
             record_cap = max(1024, self.p * 64)
-        self.rec = torch.empty(int(record_cap), dtype=torch.int32, device=self.device)
+        # pmax, sepset records and G side by side: one copy brings a small result to the host
+        pp = self.p * self.p
+        self._cuts = (8 * pp, (8 * pp + 255) // 256 * 256)
+        self._cuts += (self._cuts[1] + 4 * int(record_cap), (self._cuts[1] + 4 * int(record_cap) + 255) // 256 * 256)
+        self._out = torch.empty(self._cuts[3] + 2 * pp, dtype=torch.uint8, device=self.device)
+        self.pmax = self._out[:self._cuts[0]].view(torch.float64).view(self.p, self.p)
+        self.rec = self._out[self._cuts[1]:self._cuts[2]].view(torch.int32)
+        self.G = self._out[self._cuts[3]:].view(torch.int16).view(self.p, self.p)
+        self._rec0 = self.rec
         self.stats = _lib.GcslStats()
 
     def load(self, codes_colmajor: np.ndarray | None = None, dims: np.ndarray | None = None, codes_dev=None,
@@ -241,9 +252,18 @@ class DiscreteSolver:
 
     def to_host(self):
         n_ints = int(self.stats.n_records)
-        rec = self.rec[:n_ints].cpu().numpy() if n_ints else np.zeros(0, np.int32)
-        G = self.G.cpu().numpy().view(np.uint16)
-        pmax = self.pmax.cpu().numpy()
+        p, c = self.p, self._cuts
+        # a copy to pageable memory costs about 20 us besides its bytes: the unused records
+        # travel along where they are few (p = 23: 85 -> 37 us)
+        if self.rec is self._rec0 and 4 * self.rec.numel() <= 10 * p * p + 65536:
+            out = self._out.cpu().numpy()
+            rec = out[c[1]:c[2]].view(np.int32)[:n_ints]
+            G = out[c[3]:].view(np.uint16).reshape(p, p)
+            pmax = out[:c[0]].view(np.float64).reshape(p, p)
+        else:
+            rec = self.rec[:n_ints].cpu().numpy() if n_ints else np.zeros(0, np.int32)
+            G = self.G.cpu().numpy().view(np.uint16)
+            pmax = self.pmax.cpu().numpy()
         sep = records_to_dense(rec, n_ints, self.p, self.max_level)
         return G, sep, pmax
 

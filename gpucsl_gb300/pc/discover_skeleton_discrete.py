@@ -32,7 +32,7 @@ def discover_skeleton_gpu_discrete(
 ) -> SkeletonResult:
     torch = engine._torch()
     data = np.asarray(data)
-    codes_dev = dims_dev = None
+    codes = codes_dev = dims_dev = None
     if data.dtype.kind in "iu" or (data.dtype == np.float64 and np.all(np.isfinite(data))):
         # integer-valued categories: encoded on the device (observed values ascending)
         try:
@@ -47,11 +47,18 @@ def discover_skeleton_gpu_discrete(
         codes, dims = engine.ordinal_encode(data)
     max_dim = int(dims.max()) if dims.size else 1
     # is_debug: the bounds-checked build of the kernels (the reference compiles with -G)
-    solver = kernels.discrete_solver(num_variables, num_observations, max_level, max_dim) if kernels is not None \
-        else engine.DiscreteSolver(num_variables, num_observations, max_level, max_dim, debug=is_debug)
+    if kernels is None and codes_dev is not None and data.shape == (num_observations, num_variables):
+        # the encoder's output has the solver's layout: taken over as it is
+        solver = engine.DiscreteSolver(num_variables, num_observations, max_level, max_dim, debug=is_debug,
+                                       codes=codes_dev, dims=dims_dev)
+        codes_dev = None
+    elif kernels is not None:
+        solver = kernels.discrete_solver(num_variables, num_observations, max_level, max_dim)
+    else:
+        solver = engine.DiscreteSolver(num_variables, num_observations, max_level, max_dim, debug=is_debug)
     if codes_dev is not None:
         solver.load(codes_dev=codes_dev[:, :num_observations], dims_dev=dims_dev)
-    else:
+    elif codes is not None:
         solver.load(codes, dims)
     torch.cuda.synchronize()
     start = timer()
