@@ -321,12 +321,13 @@ def discrete_leg(flush, reps: int = 12) -> dict:
             "unit": UNIT, "ms_per_solve": round(1e3 * t, 3), "solves_timed": reps, "tests_per_solve": Ed,
             "tests_per_level": tests, "levels_run": std.raw["levels_run"],
             "l2": "flushed before every timed solve (256 MB write outside the events)",
-            "roofline": {"bound": "hbm", "kernel": "disc_test_kernel (whole solve time: a lower bound for the "
-                                                  "kernel)",
+            "roofline": {"bound": "hbm", "kernel": "whole solve (levels 0 and 1 on bit planes, further levels "
+                                                  "disc_test_kernel)",
                          "algorithmic_bytes_per_solve": int(alg_bytes), "achieved": round(achieved, 1),
                          "peak": round(peak, 1), "unit": "GB/s", "frac": round(achieved / peak, 4),
                          "peak_source": "MEASURED_PEAKS.json hbm_gbs" if "hbm_gbs" in peaks else "fallback 6.8 TB/s",
-                         "note": "codes are L2-resident after the first pass: L2-relative figure, may exceed 1"}}
+                         "note": "bytes that reading the codes for every test would take; a bit plane's read serves "
+                                 "many tests, so the figure exceeds the copy rate"}}
 
 
 def e2e_api_leg(data, solver, E: int, levels_run: int, reps: int = 10) -> dict:
