@@ -1143,16 +1143,20 @@ __device__ __forceinline__ void pmax_kept_share(const PmaxShared &S, const RTab 
     const double inf = __longlong_as_double(0x7ff0000000000000ll);
     if (threadIdx.x == 0) s_n = 0;
     __syncthreads();
+    // entries of the queue, the same in every thread (s_n itself may already hold some of a warp
+    // that is ahead in the next round when it is read after the barrier)
+    int queued = 0;
     for (int t0 = b * blockDim.x; t0 < n; t0 += nb * blockDim.x) {
         const int t = t0 + threadIdx.x;
+        bool later = false;
         if (t < n) {
             const int k = kept[t];
             const double r2 = r2min[k];
-            if (R.a != nullptr && r2 < R.rmax2 && zmin[k] == inf) pmax[k] = rt_eval(R, S.rt, sqrt(r2));
-            else s_queue[atomicAdd(&s_n, 1)] = k;
+            later = !(R.a != nullptr && r2 < R.rmax2 && zmin[k] == inf);
+            if (later) s_queue[atomicAdd(&s_n, 1)] = k;
+            else pmax[k] = rt_eval(R, S.rt, sqrt(r2));
         }
-        __syncthreads();
-        const int queued = s_n;
+        queued += __syncthreads_count(later);
         if (queued + (int)blockDim.x > PMAX_QUEUE || t0 + nb * (int)blockDim.x >= n) {  // full, or the last round
             for (int q = threadIdx.x; q < queued; q += blockDim.x) {
                 const int k = s_queue[q];
@@ -1161,8 +1165,8 @@ __device__ __forceinline__ void pmax_kept_share(const PmaxShared &S, const RTab 
                 if (r2 < 1.0) z = fmin(z, fisher_z(sqrt(r2)));  // Z increasing in rho^2 below 1
                 pmax[k] = two_sf_tab(sqrt_nm3 * z, S.sf);
             }
-            __syncthreads();
-            if (threadIdx.x == 0) s_n = 0;
+            if (threadIdx.x == 0) s_n = 0;  // (read by nobody before the barrier)
+            queued = 0;
             __syncthreads();
         }
     }
