@@ -51,9 +51,10 @@ __host__ __device__ inline int bp_group_vars(int max_dim) { return max_dim > 1 ?
 // are shifted together.  A word holds its samples in the order this gives, the same for every
 // plane, which is all that counts need.  Codes at or above the cardinality set
 // GCSL_ERR_INVALID_ARG.  The first block of a variable also stores its cardinality (1 ..
-// max_dim, the bound all buffers are sized by; a larger one sets DISC_STATUS_WIDE and the
-// solve is repeated on the general path), off[v] planes before it (d - 1 each) and foff[v]
-// values before it (d each).  LG_BLOCKS extra blocks build the ln Gamma tables.
+// max_dim, the bound all buffers are sized by; a larger one sets DISC_STATUS_WIDE, ends the
+// solve's levels, whose sepsets would come from the clamped counts, and the solve is repeated
+// on the general path), off[v] planes before it (d - 1 each) and foff[v] values before it (d
+// each).  LG_BLOCKS extra blocks build the ln Gamma tables.
 //
 // Bound by the integer pipe: 4 instructions per 4 codes and value (a ballot per sample took
 // three times as many: 66 us at p = 299, n = 99991, cardinality 2..6).
@@ -95,7 +96,10 @@ __global__ void __launch_bounds__(256) disc_planes_kernel(const uint8_t *__restr
     }
     const int d = max(1, min((int)dims[v], max_dim));
     if (chunk == 0 && threadIdx.x == 0) {
-        if (dims[v] > max_dim) set_status(st, DISC_STATUS_WIDE);
+        if (dims[v] > max_dim) {
+            set_status(st, DISC_STATUS_WIDE);
+            st->done = 1;
+        }
         card[v] = (uint8_t)d;
         off[v] = po;
         foff[v] = fo;

@@ -310,8 +310,8 @@ int gcsl_corr_tc_batch_run_flagged(const gcsl_batch_plan *plan, const int32_t *f
  *                (ld a multiple of 16; bytes in [n, ld) are ignored)
  *   dims         p uint8 observed cardinalities (discover_skeleton_discrete.py:49)
  *   max_dim      the largest entry of dims; it sizes the workspace and each level's shared-memory
- *                tables
- *                (a larger cardinality in dims sets GCSL_ERR_UNSUPPORTED)
+ *                tables (a larger cardinality in dims is solved as it is where the tables
+ *                still hold it, else the call returns GCSL_ERR_UNSUPPORTED)
  *   other arguments as for gcsl_gauss_skeleton; pmax folds every test (the reference
  *   tests every rank, discrete_ci.cu:221-244). */
 size_t gcsl_disc_workspace_bytes(int32_t p, int64_t n, int32_t max_level, int32_t max_dim);
