@@ -514,6 +514,7 @@ struct DiscWs {
     int *rows;
     unsigned long long *win;
     DiscBits bits;  // the bit-plane path's buffers when the shape takes it (planes != nullptr)
+    size_t general_bytes;  // without those
     size_t bytes;
 };
 
@@ -530,6 +531,7 @@ DiscWs carve_disc(void *ws, size_t cap, int p, long long n, int max_dim) {
     std::memset(&w.bits, 0, sizeof(w.bits));
     w.bits.max_dim = max_dim;
     w.bits.lg = c.take<double>(host::disc_lgam_doubles());
+    w.general_bytes = c.off;
     if (host::disc_bits_ok(n, p, max_dim)) {
         const size_t pl = (size_t)p * (max_dim - 1), va = (size_t)p * max_dim;
         w.bits.planes = c.take<uint32_t>(host::disc_bits_words(n, p, max_dim));
@@ -851,9 +853,12 @@ int gcsl_disc_skeleton(const uint8_t *data, int64_t ld, int64_t n, int32_t p, co
         return GCSL_ERR_INVALID_ARG;
     if (rec_pool == nullptr) rec_cap = 0;
     const DiscWs w = carve_disc(workspace, workspace_bytes, p, n, max_dim);
-    if (!workspace || w.bytes > workspace_bytes) return GCSL_ERR_WORKSPACE;
+    if (!workspace || w.general_bytes > workspace_bytes) return GCSL_ERR_WORKSPACE;
+    // the planes are a faster way, not a need: a workspace without room for them (sized for
+    // other cardinalities or fewer samples, say) takes the general path
+    const bool bits = w.bits.planes != nullptr && w.bytes <= workspace_bytes;
     DiscLevelArgs A{data, ld, n, p, dims, alpha, 0, w.adj, w.prefix, G, pmax, w.win, 0, 1024, w.st, w.bits.lg};
-    int rc = disc_solve(A, w, w.bits.planes != nullptr, max_dim, max_level, sepsets, rec_pool, rec_cap, stats,
+    int rc = disc_solve(A, w, bits, max_dim, max_level, sepsets, rec_pool, rec_cap, stats,
                         static_cast<cudaStream_t>(stream));
     if (rc == DISC_STATUS_WIDE)  // a cardinality above max_dim: the general path takes it if its tables fit
         rc = disc_solve(A, w, false, max_dim, max_level, sepsets, rec_pool, rec_cap, stats,

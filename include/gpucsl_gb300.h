@@ -312,6 +312,9 @@ int gcsl_corr_tc_batch_run_flagged(const gcsl_batch_plan *plan, const int32_t *f
  *   max_dim      the largest entry of dims; it sizes the workspace and each level's shared-memory
  *                tables (a larger cardinality in dims is solved as it is where the tables
  *                still hold it, else the call returns GCSL_ERR_UNSUPPORTED)
+ *   workspace    gcsl_disc_workspace_bytes(p, n, max_level, max_dim) bytes; one that lacks only
+ *                the bit planes of levels 0 and 1 (the size for max_dim = 1) is taken too, and
+ *                these levels then count every test's table on its own
  *   other arguments as for gcsl_gauss_skeleton; pmax folds every test (the reference
  *   tests every rank, discrete_ci.cu:221-244). */
 size_t gcsl_disc_workspace_bytes(int32_t p, int64_t n, int32_t max_level, int32_t max_dim);

@@ -1,5 +1,6 @@
 """The C entry point of the discrete solve with a dense separation-set buffer, against the C
-oracle: a cardinality above the announced maximum must leave nothing of its first attempt behind."""
+oracle: a cardinality above the announced maximum must leave nothing of its first attempt behind,
+and a workspace without room for the optional buffers is enough."""
 import ctypes as ct
 
 import numpy as np
@@ -49,3 +50,18 @@ def test_sets_of_a_repeated_solve(cuda):
     rc, got = run_entry(cuda, codes, dims, 0.05, 1, 2)
     assert rc == 0
     assert_parity(got, oracle_discrete(codes, dims, 0.05, 1))
+
+
+def test_workspace_of_the_general_path(cuda):
+    """The bit planes are optional: a workspace that holds the other buffers is accepted."""
+    from test_gpu_disc_bits import dependent_codes
+    from gpucsl_gb300 import _lib
+
+    codes, dims = dependent_codes(40, 1500, 4, 77)
+    small = int(_lib.lib().gcsl_disc_workspace_bytes(40, 1500, 2, 1))  # no planes for constant columns
+    assert small < int(_lib.lib().gcsl_disc_workspace_bytes(40, 1500, 2, 4))
+    ref = oracle_discrete(codes, dims, 0.05, 2)
+    rc, got = run_entry(cuda, codes, dims, 0.05, 2, 4, small)
+    assert rc == 0
+    assert_parity(got, ref)
+    assert run_entry(cuda, codes, dims, 0.05, 2, 4, small - 1)[0] == _lib.GCSL_ERR_WORKSPACE
