@@ -45,33 +45,32 @@ __host__ __device__ inline long long bp_words(long long n) {
 __host__ __device__ inline int bp_group_vars(int max_dim) { return max_dim > 1 ? BP_GROUP / (max_dim - 1) : BP_GROUP; }
 
 // ------------------------------------------------------------------ bit planes
-// Block (chunk, v): planes of variable v.  A lane takes 32 samples (two 16-byte loads) and
+// Item (chunk, v): planes of variable v.  A lane takes 32 samples (two 16-byte loads) and
 // makes one word of every plane: four codes at a time, a byte of (w ^ aaaa) + 0x7f.. has its
 // high bit clear exactly where the code is a (codes below 128), and the eight steps' bits
 // are shifted together.  A word holds its samples in the order this gives, the same for every
 // plane, which is all that counts need.  Codes at or above the cardinality set
-// GCSL_ERR_INVALID_ARG.  The first block of a variable also stores its cardinality (1 ..
+// GCSL_ERR_INVALID_ARG.  The first item of a variable also stores its cardinality (1 ..
 // max_dim, the bound all buffers are sized by; a larger one sets DISC_STATUS_WIDE, ends the
 // solve's levels, whose sepsets would come from the clamped counts, and the solve is repeated
 // on the general path), off[v] planes before it (d - 1 each) and foff[v] values before it (d
-// each).  LG_BLOCKS extra blocks build the ln Gamma tables.
+// each).  LG_BLOCKS extra items build the ln Gamma tables.
 //
 // Bound by the integer pipe: 4 instructions per 4 codes and value (a ballot per sample took
 // three times as many: 66 us at p = 299, n = 99991, cardinality 2..6).
-__global__ void __launch_bounds__(256) disc_planes_kernel(const uint8_t *__restrict__ data, long long ld, long long n,
-                                                          int p, const uint8_t *__restrict__ dims, int max_dim,
-                                                          int chunks, uint32_t *__restrict__ planes, long long words,
-                                                          uint8_t *__restrict__ card, int *__restrict__ off,
-                                                          int *__restrict__ foff, double *__restrict__ lg,
-                                                          DevState *st) {
-    if ((int)blockIdx.x >= chunks * p) {
-        lgam_build(lg, (int)blockIdx.x - chunks * p);
+__device__ __forceinline__ void planes_item(int item, const uint8_t *__restrict__ data, long long ld, long long n,
+                                            int p, const uint8_t *__restrict__ dims, int max_dim, int chunks,
+                                            uint32_t *__restrict__ planes, long long words, uint8_t *__restrict__ card,
+                                            int *__restrict__ off, int *__restrict__ foff, double *__restrict__ lg,
+                                            DevState *st) {
+    __shared__ int s_sum[8][2];
+    if (item >= chunks * p) {
+        lgam_build(lg, item - chunks * p);
         return;
     }
-    const int v = (int)blockIdx.x / chunks, chunk = (int)blockIdx.x - v * chunks;
+    const int v = item / chunks, chunk = item - v * chunks;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // planes and values before v
-    __shared__ int s_sum[8][2];
     int po = 0, fo = 0;
     for (int u = threadIdx.x; u < v; u += blockDim.x) {
         const int d = max(1, min((int)dims[u], max_dim));
@@ -143,6 +142,19 @@ __global__ void __launch_bounds__(256) disc_planes_kernel(const uint8_t *__restr
     }
     if (dv > 128) bad = 0;  // more than max_dim values: the general path checks them
     if (__any_sync(GCSL_FULL_MASK, bad != 0) && lane == 0) set_status(st, GCSL_ERR_INVALID_ARG);
+}
+
+// One item a block, or with a cap on the resident blocks several.
+__global__ void __launch_bounds__(256) disc_planes_kernel(const uint8_t *__restrict__ data, long long ld, long long n,
+                                                          int p, const uint8_t *__restrict__ dims, int max_dim,
+                                                          int chunks, uint32_t *__restrict__ planes, long long words,
+                                                          uint8_t *__restrict__ card, int *__restrict__ off,
+                                                          int *__restrict__ foff, double *__restrict__ lg,
+                                                          DevState *st) {
+    for (int item = (int)blockIdx.x; item < chunks * p + LG_BLOCKS; item += (int)gridDim.x) {
+        planes_item(item, data, ld, n, p, dims, max_dim, chunks, planes, words, card, off, foff, lg, st);
+        __syncthreads();  // its shared sums are read
+    }
 }
 
 // ------------------------------------------------------------ counts of a block
@@ -777,11 +789,15 @@ cudaError_t launch_disc_bits_level0(const DiscBits &b, const DiscLevelArgs &A, i
     const int chunks = (int)(want < 1 ? 1 : want > most ? most : want);
     cudaError_t e = cudaMemsetAsync(b.counts, 0, (size_t)ldc * ldc * sizeof(uint32_t), s);
     if (e != cudaSuccess) return e;
-    disc_planes_kernel<<<chunks * p + LG_BLOCKS, 256, 0, s>>>(A.data, A.ld, A.n, p, A.dims, b.max_dim, chunks, b.planes,
+    // room left on every SM for concurrent solves: at most `cap` blocks of 256 threads on each
+    const int cap = blocks_per_sm_cap();
+    const int items = chunks * p + LG_BLOCKS;
+    disc_planes_kernel<<<cap > 0 ? std::min(items, num_sms * cap) : items, 256, 0, s>>>(A.data, A.ld, A.n, p, A.dims, b.max_dim, chunks, b.planes,
                                                               words, b.card, b.off, b.foff, b.lg, A.st);
-    disc_pair_counts_kernel<<<num_sms * 2, 256, 0, s>>>(b.planes, words, b.off, p, b.counts, ldc);
+    disc_pair_counts_kernel<<<num_sms * (cap == 1 ? 1 : 2), 256, 0, s>>>(b.planes, words, b.off, p, b.counts, ldc);
     const long long pairs = (long long)p * (p + 1) / 2, lb = (pairs + BP_L0_GROUPS - 1) / BP_L0_GROUPS;
-    disc_level0_kernel<<<(unsigned)std::min(lb, num_sms * 16ll), BP_L0_THREADS, 0, s>>>(
+    const long long l0_per_sm = cap > 0 ? std::min(16, cap * (256 / BP_L0_THREADS)) : 16;
+    disc_level0_kernel<<<(unsigned)std::min(lb, num_sms * l0_per_sm), BP_L0_THREADS, 0, s>>>(
         b.counts, ldc, p, b.card, b.off, b.foff, (uint32_t)A.n, b.full, b.inv, ldf, A.alpha, b.lg, A.G, A.pmax, A.st, A.order);
     note_launch(3);
     return note_error("discrete level 0 launch", cudaGetLastError());

@@ -80,7 +80,8 @@ int gcsl_set_test_precision(int32_t mode);
  * release library returns GCSL_ERR_UNSUPPORTED. */
 int gcsl_debug_set_work_order(uint64_t seed);
 /* Serving (no reference counterpart): caps the resident blocks per SM of the discrete
- * test kernel (a grid-stride kernel that otherwise fills every SM for the whole level)
+ * kernels that otherwise fill every SM for the whole level (blocks of 256 threads, or as many
+ * threads in smaller ones; a test of the general path from level 1 on takes a block of 512),
  * launched by the calling thread; 0 = as many as fit.  A server that runs discrete
  * solves next to other work sets it so that the other work finds room on every SM.
  * Results do not depend on it. */
