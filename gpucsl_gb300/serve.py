@@ -89,13 +89,13 @@ class Response:
 
 
 def gaussian_footprint(p: int, n: int, max_level: int) -> int:
-    """Device bytes of one Gaussian request in a batch: samples (FP32), correlation
-    workspace (7 BF16 digit planes + int64 partials), C, skeleton, pmax, the level-loop
-    slice and a record pool."""
-    p_pad = (p + 127) // 128 * 128
-    n_pad = (n + 31) // 32 * 32
-    return (4 * n * p + 14 * p_pad * n_pad + 16 * p_pad * p_pad + 8 * p * p + 2 * p * p + 8 * p * p
-            + (4 + 8 + 8 + 2) * p * p + 4 * max(1024, 64 * p) + 4096)
+    """Device bytes of one Gaussian request: samples (FP32), the correlation's workspace (7 BF16
+    digit planes, int64 partial sums of every K split), C, skeleton, pmax, a record pool and the
+    level loop's state in a batch or workspace alone, whichever is larger."""
+    L = _lib.lib()
+    return (4 * n * p + int(L.gcsl_corr_tc_workspace_bytes(n, p)) + (8 + 2 + 8) * p * p
+            + max(int(L.gcsl_gauss_state_bytes(p)), int(L.gcsl_gauss_workspace_bytes(p, max_level)))
+            + 4 * max(1024, 64 * p) + 4096)
 
 
 def discrete_footprint(p: int, n: int, max_level: int, max_dim: int) -> int:
