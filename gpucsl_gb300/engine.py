@@ -202,9 +202,16 @@ class DiscreteSolver:
         L = _lib.lib(self.debug)
         ws = int(L.gcsl_disc_workspace_bytes(self.p, self.n, self.max_level, self.max_dim))
         self.workspace = torch.empty(ws, dtype=torch.uint8, device=self.device)
-        if codes is not None and (tuple(codes.shape) != (self.p, self.ld) or not codes.is_contiguous()
-                                  or codes.data_ptr() % 16):
-            raise ValueError("codes must be a contiguous (p, n rounded up to 16) tensor on a 16-byte boundary")
+        # the kernels read both as they are
+        def checked(name, t, shape, what):
+            if t is not None and (t.dtype != torch.uint8 or t.device != self.workspace.device
+                                  or tuple(t.shape) != shape or not t.is_contiguous()):
+                raise ValueError(f"{name} must be a contiguous {what} uint8 tensor on the solver's device")
+
+        checked("codes", codes, (self.p, self.ld), "(p, n rounded up to 16)")
+        checked("dims", dims, (self.p,), "(p,)")
+        if codes is not None and codes.data_ptr() % 16:
+            raise ValueError("codes must start on a 16-byte boundary")
         self.data = torch.zeros((self.p, self.ld), dtype=torch.uint8, device=self.device) if codes is None else codes
         self.dims = torch.empty(self.p, dtype=torch.uint8, device=self.device) if dims is None else dims
         if record_cap is None:
