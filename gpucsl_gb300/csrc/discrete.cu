@@ -249,7 +249,9 @@ __device__ double table_chi2(const uint32_t *sm_tab, int dim_s, int di, int dj, 
         uint32_t ma, mb;
         marginals(k, s, ma, mb);
         if (ma == 0 || mb == 0) continue;
-        const long long e = (long long)ma * mb, q = (long long)sm_tab[k] * s_mt[s] - e;
+        // unsigned: a product of two counts of up to 2^32 samples; |q| is at most a quarter of it
+        const unsigned long long e = (unsigned long long)ma * mb;
+        const long long q = (long long)((unsigned long long)sm_tab[k] * s_mt[s] - e);
         chi += (double)q * (double)q / ((double)e * (double)s_mt[s]);
     }
 #pragma unroll
