@@ -27,8 +27,8 @@
 // a pass took 296 us.
 // The barriers' waits have a time limit, so a step has to be short against it: where the sum of
 // cubed degrees (a bound on a step's work) is above OR_MAX_WORK, the same steps run as separate
-// kernels.  Close to the line the two cost about the same (1000 vertices of degree 39: 218 us
-// in one kernel; of degree 42: 277 us, 50 of them for the list and the check).
+// kernels.  Close to the line the two cost about the same (1000 vertices of degree 39: 169 us
+// in one kernel; of degree 60, in separate ones: 152).
 #include "common.cuh"
 #include "gauss_dev.cuh"
 
@@ -38,6 +38,11 @@ constexpr unsigned long long OR_NONE = 0xffffffffffffffffull;
 constexpr unsigned long long OR_MAX_WORK = 1ull << 26;
 constexpr long long OR_WAIT_NS = 4000000000ll;  // a barrier's limit
 constexpr int OR_MAX_PASSES = 1 << 20;          // of one cooperative launch
+// Warps per row of a dense graph's neighbours (for_edges), as far as the SMs hold them: with one,
+// 300 vertices of degree 150 kept 38 blocks busy.  One kernel (at most a block an SM) against
+// one warp a row: 100 vertices of degree 40: 178 -> 85 us, of degree 5: 66 -> 67; separate kernels:
+// 300 of degree 150: 1061 -> 197 us, 1000 of degree 200: 1565 -> 374.
+constexpr int OR_SHARE = 4, OR_SHARE_STEPS = 16;
 
 enum OrStatus { OR_UNFINISHED = 0, OR_DONE = 1 };
 
@@ -65,15 +70,18 @@ __device__ __forceinline__ bool arc(const uint8_t *D, int p, int a, int b) {
 }
 
 // f(a, b, list of a, degree of a, lane of the group, group mask) for every directed pair
-// (a, b) of adjacent vertices: warp per row a, eight lanes per neighbour b.
+// (a, b) of adjacent vertices: eight lanes per neighbour b; warp per row a, or with more warps
+// than rows several per row, which take turns in its neighbours.
 template <typename F>
 __device__ __forceinline__ void for_edges(const int *adj, int p, int warp, int warps, F f) {
     const int lane = threadIdx.x & 31, sub = lane & 7;
     const unsigned group = 0xffu << (lane & 24);
-    for (int a = warp; a < p; a += warps) {
+    const int share = warps > p ? warps / p : 1, rows = warps / share, part = warp / rows;
+    if (part >= share) return;
+    for (int a = warp - part * rows; a < p; a += rows) {
         const int *ra = adj + (size_t)a * p;
         const int da = __ldcg(ra);
-        for (int t = lane >> 3; t < da; t += 4) f(a, __ldcg(ra + 1 + t), ra, da, sub, group);
+        for (int t = 4 * part + (lane >> 3); t < da; t += 4 * share) f(a, __ldcg(ra + 1 + t), ra, da, sub, group);
     }
 }
 
@@ -328,12 +336,13 @@ cudaError_t orient_edges(const uint16_t *S, int p, const int *sep, int L, uint8_
     unsigned long long *key = reinterpret_cast<unsigned long long *>(w + al(pp * sizeof(int)) + al(pp));
     OrCtl *ctl = reinterpret_cast<OrCtl *>(w + al(pp * sizeof(int)) + al(pp) + al(pp * 8));
     const int rows_blocks = (p + 7) / 8;
+    const int step_blocks = std::max(rows_blocks, std::min(rows_blocks * OR_SHARE_STEPS, num_sms * 8));
     cudaError_t e = cudaMemsetAsync(ctl, 0, sizeof(OrCtl), s);
     if (e != cudaSuccess) return e;
     void *args[] = {&S, &p, &sep, &L, &adj, &P, &D, &key, &ctl};
     // at most one block an SM: all resident
     e = cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(orient_kernel),
-                                    dim3((unsigned)std::min(rows_blocks, num_sms)), dim3(256), args, 0, s);
+                                    dim3((unsigned)std::min(rows_blocks * OR_SHARE, num_sms)), dim3(256), args, 0, s);
     if (e == cudaErrorCooperativeLaunchTooLarge) {  // fewer SMs than the device's for this context
         cudaGetLastError();
         host_words[0] = OR_UNFINISHED;
@@ -357,7 +366,7 @@ cudaError_t orient_edges(const uint16_t *S, int p, const int *sep, int L, uint8_
         ++n;
         if ((e = cudaMemsetAsync(&ctl->changed, 0, sizeof(int), s)) != cudaSuccess) return e;
         for (int step = first; step < 8; ++step)
-            orient_step_kernel<<<rows_blocks, 256, 0, s>>>(S, p, sep, L, adj, P, D, key, ctl, step);
+            orient_step_kernel<<<step_blocks, 256, 0, s>>>(S, p, sep, L, adj, P, D, key, ctl, step);
         note_launch(8 - first);
         if ((e = cudaMemcpyAsync(host_words, &ctl->changed, sizeof(int), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
             (e = cudaStreamSynchronize(s)) != cudaSuccess)
