@@ -337,12 +337,14 @@ cudaError_t orient_edges(const uint16_t *S, int p, const int *sep, int L, uint8_
     OrCtl *ctl = reinterpret_cast<OrCtl *>(w + al(pp * sizeof(int)) + al(pp) + al(pp * 8));
     const int rows_blocks = (p + 7) / 8;
     const int step_blocks = std::max(rows_blocks, std::min(rows_blocks * OR_SHARE_STEPS, num_sms * 8));
+    int coop_blocks = std::min(rows_blocks * OR_SHARE, num_sms);
+    if (coop_blocks < 2 * rows_blocks) coop_blocks = std::min(rows_blocks, num_sms);  // no two warps for every row
     cudaError_t e = cudaMemsetAsync(ctl, 0, sizeof(OrCtl), s);
     if (e != cudaSuccess) return e;
     void *args[] = {&S, &p, &sep, &L, &adj, &P, &D, &key, &ctl};
     // at most one block an SM: all resident
     e = cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(orient_kernel),
-                                    dim3((unsigned)std::min(rows_blocks * OR_SHARE, num_sms)), dim3(256), args, 0, s);
+                                    dim3((unsigned)coop_blocks), dim3(256), args, 0, s);
     if (e == cudaErrorCooperativeLaunchTooLarge) {  // fewer SMs than the device's for this context
         cudaGetLastError();
         host_words[0] = OR_UNFINISHED;
