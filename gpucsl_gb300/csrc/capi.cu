@@ -54,9 +54,12 @@ void disc_level_caps(int cap_full, int max_dim, int L, int &table_cap, int &part
 cudaError_t launch_disc_tests(const DiscLevelArgs &A, int num_sms, cudaStream_t s);
 cudaError_t launch_disc_validate(const uint8_t *data, long long ld, long long n, int p, const uint8_t *dims,
                                  double *lg, DevState *st, int num_sms, cudaStream_t s);
-cudaError_t launch_disc_plan(const int *adj, int p, int L, int group, const uint8_t *dims, long long *w,
-                             long long *prefix, long long *tasks, int *rows, DevState *st, cudaStream_t s);
+cudaError_t launch_disc_plan(const int *adj, int p, int L, int group, int max_dim, long long n, const int *planes,
+                             const uint8_t *dims, long long *w, long long *prefix, long long *tasks, int *rows,
+                             DevState *st, cudaStream_t s);
 bool disc_bits_ok(long long n, int p, int max_dim);
+bool disc_bits_level0(long long n, int p, int max_dim);
+bool disc_bits_level1(int max_dim);
 size_t disc_bits_words(long long n, int p, int max_dim);
 int disc_bits_group(int max_dim);
 size_t disc_lgam_doubles();
@@ -532,12 +535,14 @@ DiscWs carve_disc(void *ws, size_t cap, int p, long long n, int max_dim) {
     w.bits.max_dim = max_dim;
     w.bits.lg = c.take<double>(host::disc_lgam_doubles());
     w.general_bytes = c.off;
-    if (host::disc_bits_ok(n, p, max_dim)) {
+    if (host::disc_bits_ok(n, p, max_dim) && host::disc_bits_level0(n, p, max_dim)) {
         const size_t pl = (size_t)p * (max_dim - 1), va = (size_t)p * max_dim;
         w.bits.planes = c.take<uint32_t>(host::disc_bits_words(n, p, max_dim));
         w.bits.counts = c.take<uint32_t>(pl * pl);
-        w.bits.full = c.take<uint32_t>(va * va);
-        w.bits.inv = c.take<double>(va * va);
+        if (host::disc_bits_level1(max_dim)) {
+            w.bits.full = c.take<uint32_t>(va * va);
+            w.bits.inv = c.take<double>(va * va);
+        }
         w.bits.card = c.take<uint8_t>((size_t)p);
         w.bits.off = c.take<int>((size_t)p + 1);
         w.bits.foff = c.take<int>((size_t)p + 1);
@@ -546,7 +551,7 @@ DiscWs carve_disc(void *ws, size_t cap, int p, long long n, int max_dim) {
     return w;
 }
 
-// One discrete solve; with bits, levels 0 and 1 run on bit planes.
+// One discrete solve; with bits, level 0 runs on bit planes and level 1 may.
 int disc_solve(DiscLevelArgs A, const DiscWs &w, bool bits, int max_dim, int max_level, int *sepsets, int *rec_pool,
                long long rec_cap, gcsl_stats *stats, cudaStream_t s) {
     const int sms = device_sms(), p = A.p;
@@ -572,16 +577,17 @@ int disc_solve(DiscLevelArgs A, const DiscWs &w, bool bits, int max_dim, int max
     HostCtl *hc = host_ctl();
     if (!hc) return GCSL_ERR_DEVICE;
     auto disc_level = [&](int level) -> cudaError_t {
-        const bool planes = bits && level == 1;
+        const bool planes = bits && level == 1 && w.bits.full != nullptr;
         cudaError_t e2 = host::launch_compact(A.G, p, w.adj, nullptr, w.st, level, nullptr, s);
         if (e2 == cudaSuccess)
-            e2 = host::launch_disc_plan(w.adj, p, level, planes ? host::disc_bits_group(max_dim) : 0, A.dims,
-                                        w.weights, w.prefix, w.tasks, w.rows, w.st, s);
+            e2 = host::launch_disc_plan(w.adj, p, level, planes ? host::disc_bits_group(max_dim) : 0, max_dim, A.n,
+                                        w.bits.off, A.dims, w.weights, w.prefix, w.tasks, w.rows, w.st, s);
         DiscLevelArgs B = A;
         B.level = level;
         host::disc_level_caps(cap, max_dim, level, B.table_cap, B.part_cap);
-        if (e2 == cudaSuccess)
-            e2 = planes ? host::launch_disc_bits_level1(w.bits, B, w.tasks, w.rows, sms, s) : host::launch_disc_tests(B, sms, s);
+        B.routed = planes;
+        if (e2 == cudaSuccess && planes) e2 = host::launch_disc_bits_level1(w.bits, B, w.tasks, w.rows, sms, s);
+        if (e2 == cudaSuccess) e2 = host::launch_disc_tests(B, sms, s);
         if (e2 == cudaSuccess)
             e2 = host::launch_disc_finalize(w.adj, p, level, A.G, w.win, sepsets, max_level, rec_pool, rec_cap, w.st,
                                             sms, s);

@@ -154,7 +154,7 @@ struct DevState {
     int32_t last_level;                      // highest level whose tests ran
     int32_t n_kept;                          // pairs kept at level 0 (Gaussian)
     int32_t debug_site;                      // first failed check of the debug build (GCSL_DCHECK_*), 0 if none
-    int32_t reserved_;
+    int32_t disc_route;                      // level 1 of a discrete solve: 0 on bit planes, 1 a table a test
     int32_t max_degree[GCSL_MAX_LEVELS];     // max compacted degree at level start
     unsigned long long edges[GCSL_MAX_LEVELS];
     unsigned long long tests[GCSL_MAX_LEVELS];
@@ -214,6 +214,7 @@ struct DiscLevelArgs {
     int part_cap;             // strata of the per-stratum statistic buffer (after the table)
     DevState *st;
     const double *lg;         // ln Gamma tables of the p-value series
+    bool routed = false;      // launched beside the bit-plane kernel: st->disc_route says which of the two runs
     unsigned long long order = 0;  // work order of the debug build (0: launch order)
 };
 
@@ -223,7 +224,7 @@ struct DiscBits {
     int max_dim;
     uint32_t *planes;  // one bit plane per value but the last of every variable
     uint32_t *counts;  // counts of all pairs of planes
-    uint32_t *full;    // counts of all pairs of values
+    uint32_t *full;    // counts of all pairs of values (null: level 1 does not run on planes)
     double *inv;       // their reciprocals (0 for an empty pair)
     uint8_t *card;     // cardinalities, at most max_dim
     int *off, *foff;   // planes / values before each variable

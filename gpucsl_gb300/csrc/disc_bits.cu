@@ -34,6 +34,7 @@ namespace gcsl {
 constexpr int BP_SIDE = 4;         // planes on each side of a warp's block
 constexpr int BP_GROUP = 24;       // planes of a neighbour group of a level-1 task
 constexpr int BP_LANES = 8;        // lanes that share one test's statistic
+constexpr int BP_LEVEL1_DIM = 10;  // level 1: values of a variable up to which planes may pay
 constexpr int BP_ROUND = 64;       // words of one pass of a warp (2 a lane): slices are multiples
 
 // Words of a plane: whole passes, zero past the samples.
@@ -144,13 +145,20 @@ __device__ __forceinline__ void planes_item(int item, const uint8_t *__restrict_
     if (__any_sync(GCSL_FULL_MASK, bad != 0) && lane == 0) set_status(st, GCSL_ERR_INVALID_ARG);
 }
 
-// One item a block, or with a cap on the resident blocks several.
+// One item a block, or with a cap on the resident blocks several.  The blocks also clear the pair
+// counts (`cells` words on a 16-byte boundary), which the next kernel adds to.
 __global__ void __launch_bounds__(256) disc_planes_kernel(const uint8_t *__restrict__ data, long long ld, long long n,
                                                           int p, const uint8_t *__restrict__ dims, int max_dim,
                                                           int chunks, uint32_t *__restrict__ planes, long long words,
                                                           uint8_t *__restrict__ card, int *__restrict__ off,
                                                           int *__restrict__ foff, double *__restrict__ lg,
+                                                          uint32_t *__restrict__ counts, long long cells,
                                                           DevState *st) {
+    const long long thread = (long long)blockIdx.x * blockDim.x + threadIdx.x,
+                    threads = (long long)gridDim.x * blockDim.x;
+    for (long long k = thread; k < cells / 4; k += threads)
+        reinterpret_cast<uint4 *>(counts)[k] = make_uint4(0u, 0u, 0u, 0u);
+    if (thread < cells % 4) counts[cells - 1 - thread] = 0u;
     for (int item = (int)blockIdx.x; item < chunks * p + LG_BLOCKS; item += (int)gridDim.x) {
         planes_item(item, data, ld, n, p, dims, max_dim, chunks, planes, words, card, off, foff, lg, st);
         __syncthreads();  // its shared sums are read
@@ -351,8 +359,9 @@ struct PairTable {
 };
 
 // Level 0, a group of BP_LANES lanes per pair (vi >= vj): its full table F (all values, both
-// triangles, the counts of single values on the diagonal) with the reciprocals, for level 1,
-// and its test.  The last row and column of a table come from the counts of single values.
+// triangles, the counts of single values on the diagonal) with the reciprocals, for level 1
+// (where `full` is given), and its test.  The last row and column of a table come from the counts
+// of single values.
 // p-values are evaluated a thread per test at the end of a round.
 constexpr int BP_L0_THREADS = 128, BP_L0_GROUPS = BP_L0_THREADS / BP_LANES;
 __global__ void __launch_bounds__(BP_L0_THREADS) disc_level0_kernel(
@@ -412,11 +421,13 @@ __global__ void __launch_bounds__(BP_L0_THREADS) disc_level0_kernel(
             int df = -1;  // no p-value to evaluate
             if (vi == vj) {
                 for (int a = gl; a < di; a += BP_LANES) {
+                    if (full == nullptr) break;
                     full[(size_t)(fi + a) * ldf + fi + a] = nr[a];
                     inv[(size_t)(fi + a) * ldf + fi + a] = nr[a] ? 1.0 / (double)nr[a] : 0.0;
                 }
             } else {
                 group_cells(1, di, dj, gl, [&](int, int a, int b) {
+                    if (full == nullptr) return;
                     const uint32_t c = tab[a * dj + b];
                     const double r = c ? 1.0 / (double)c : 0.0;
                     full[(size_t)(fi + a) * ldf + fj + b] = c;
@@ -539,6 +550,7 @@ __global__ void __launch_bounds__(BP_L1_THREADS, 512 / BP_L1_THREADS) disc_bits_
         if (blockIdx.x == 0 && threadIdx.x == 0) st->done = 1;
         return;
     }
+    if (st->disc_route != 0) return;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         st->last_level = 1;
         st->tests[1] = (unsigned long long)A.prefix[A.p];
@@ -775,6 +787,24 @@ bool disc_bits_ok(long long n, int p, int max_dim) {
            (long long)p * (max_dim - 1) * bp_words(n) < (1ll << 32);
 }
 
+// Whether level 0 is counted on planes (three kernels, the first of them with the planes' words
+// rounded up to whole passes) or with a table for each pair (two, cheap while the pairs are few).
+// Where level 1 may follow on planes the lines lie where a solve of both levels takes the same,
+// in the median over samples and graphs (planes with the better level 1, tables, us): 4 values:
+// 16 variables 138, 133, 23 variables 185, 235; 8 values: 32 variables 349, 333; 10 values: 48
+// variables 644, 604, 80 variables 1018, 1028.  With more values level 1 has its tables, and
+// level 0 alone takes, 12 values, n = 2000: 40 variables 141, 98, 100 variables 168, 205; 16
+// values, 200 variables: n = 10000 624, 644, n = 50000 1416, 928.
+bool disc_bits_level0(long long n, int p, int max_dim) {
+    if (max_dim <= 8) return p >= 10 + 4 * (max_dim - 2);
+    return max_dim <= BP_LEVEL1_DIM ? p >= 64 : p >= 128 && n <= 16384;
+}
+
+// Whether level 1 may run on planes (the plan of the level decides, disc_level1_route).  With 12
+// values it never paid (all tests of 23 .. 200 variables: 1.08 to 3.2 times the tables' time), with
+// 10 it does where the graph is dense and n small (32 variables, n = 1000: 1521, 2562 us).
+bool disc_bits_level1(int max_dim) { return max_dim <= BP_LEVEL1_DIM; }
+
 int disc_bits_group(int max_dim) { return bp_group_vars(max_dim); }
 
 size_t disc_lgam_doubles() { return 2 * LG_TERMS; }
@@ -787,13 +817,12 @@ cudaError_t launch_disc_bits_level0(const DiscBits &b, const DiscLevelArgs &A, i
     // 256 words a block and pass; about eight blocks per SM over all variables
     const long long want = (8ll * num_sms + p - 1) / p, most = (words + 255) / 256;
     const int chunks = (int)(want < 1 ? 1 : want > most ? most : want);
-    cudaError_t e = cudaMemsetAsync(b.counts, 0, (size_t)ldc * ldc * sizeof(uint32_t), s);
-    if (e != cudaSuccess) return e;
     // room left on every SM for concurrent solves: at most `cap` blocks of 256 threads on each
     const int cap = blocks_per_sm_cap();
     const int items = chunks * p + LG_BLOCKS;
     disc_planes_kernel<<<cap > 0 ? std::min(items, num_sms * cap) : items, 256, 0, s>>>(A.data, A.ld, A.n, p, A.dims, b.max_dim, chunks, b.planes,
-                                                              words, b.card, b.off, b.foff, b.lg, A.st);
+                                                              words, b.card, b.off, b.foff, b.lg, b.counts,
+                                                              (long long)ldc * ldc, A.st);
     disc_pair_counts_kernel<<<num_sms * (cap == 1 ? 1 : 2), 256, 0, s>>>(b.planes, words, b.off, p, b.counts, ldc);
     const long long pairs = (long long)p * (p + 1) / 2, lb = (pairs + BP_L0_GROUPS - 1) / BP_L0_GROUPS;
     const long long l0_per_sm = cap > 0 ? std::min(16, cap * (256 / BP_L0_THREADS)) : 16;

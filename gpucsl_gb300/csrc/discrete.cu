@@ -5,16 +5,16 @@
 //   p-value        disc_stat.cuh         (reference: helpers/math_helpers.cu:54-175)
 //   write-back     disc_finalize_kernel  (reference: helpers/graph_helpers.cu:81-101)
 //
-// Levels 0 and 1 of tables of up to 16 values per variable run on bit planes (disc_bits.cu);
-// the kernels here take the other levels and wider tables.
+// Levels 0 and 1 run on bit planes (disc_bits.cu) where those are faster (disc_bits_level0,
+// disc_level1_route); the kernels here take the other levels, and these ones otherwise.
 //
 // One CTA evaluates one test at a time (grid-stride over the level's flattened test
 // list): the l+2 uint8 columns are streamed with 16-byte loads and counted into a
 // shared-memory table N[s][a][b] (several copies when the table is small, so that
-// lanes of a warp rarely hit the same counter), the copies are merged, each stratum's
-// marginals and (a, b)-ordered chi^2 partial sum are formed by one thread, and thread 0
-// adds the strata in ascending order and evaluates the p-value.  Counts are exact
-// integers; the chi^2 order is fixed, so results do not depend on scheduling.
+// lanes of a warp rarely hit the same counter), the copies are merged, the threads take the
+// table's cells one each at a time (table_chi2; tables wider than 32 values one stratum each, in
+// the oracle's order), and a warp evaluates the p-value.  Counts are exact integers; the order of
+// the chi^2 sum follows from the block's size alone, so results do not depend on scheduling.
 //
 // As in the reference every rank of every direction is tested (discrete_ci.cu:221-244
 // has no effective early exit) and pmax folds all of them.  The removing test with the
@@ -303,6 +303,7 @@ __global__ void __launch_bounds__(DISC_THREADS) disc_test_kernel(DiscLevelArgs A
     double *s_part = reinterpret_cast<double *>(sm_tab + ((A.table_cap + 1) & ~1));
     __shared__ int s_trusted;
     DevState *st = A.st;
+    pdl_wait();  // every thread: what follows this kernel must find the one before it complete
     if (threadIdx.x == 0) {
         s_bad = 0;
         // codes checked in range for this solve: disc_validate_kernel (or the plane writer) ran
@@ -318,6 +319,7 @@ __global__ void __launch_bounds__(DISC_THREADS) disc_test_kernel(DiscLevelArgs A
             if (blockIdx.x == 0 && threadIdx.x == 0) st->done = 1;
             return;
         }
+        if (A.routed && st->disc_route == 0) return;
         if (blockIdx.x == 0 && threadIdx.x == 0) st->last_level = L;
     }
     const long long total = (L == 0) ? (long long)A.p * (A.p - 1) / 2 : A.prefix[A.p];
@@ -480,17 +482,41 @@ __global__ void __launch_bounds__(256) disc_validate_kernel(const uint8_t *__res
     if (__any_sync(GCSL_FULL_MASK, bad) && (threadIdx.x & 31) == 0) set_status(st, GCSL_ERR_INVALID_ARG);
 }
 
+// Level 1: 0 when its `tests` are faster on bit planes, 1 when a table for each is.  Times in
+// microseconds of both ways, from what bounds each.  Planes: the longest task (`task` passes of
+// 64 words by one block, which waits for its loads) or all tasks' passes (`passes`), and the
+// statistics: their cells, or one test's series, whose terms a thread adds one by one.  Tables:
+// one test's pass over the samples, or all tests'.
+//
+// The constants fit both ways' times over 594 problems of 2 .. 10 values, 10 .. 300 variables,
+// 200 .. 500000 samples and sparse to complete graphs: by this rule a solve takes 0.4 % longer
+// than by the better way on average, 24 % in the worst of them.  Levels 0 and 1 on planes and by
+// tables: 8 values, 23 variables, n = 200000, 354 tests: 2176, 251 us; 40 variables, n = 10000,
+// all 59280 tests: 890, 1904 us.
+__device__ __forceinline__ int disc_level1_route(float tests, float task, float passes, int max_dim, float mean_planes,
+                                                 float n) {
+    const float d = (float)max_dim, m = mean_planes + 1.0f;
+    const float planes = 8.0f + fmaxf(0.14f * task, passes * (1.0f / 4600.0f)) +
+                         fmaxf(1.2e-5f * tests * m * m * m, 0.26f * d * d * d);
+    const float tables = 15.0f + fmaxf(1.7e-4f * n, tests * (0.05f + 7.3e-7f * n));
+    return planes < tables ? 0 : 1;
+}
+
 // One block plans a level: per-row test counts deg C(deg - 1, L) and their exclusive prefix,
 // the edge and test totals, and with group > 0 the bit-plane path's tasks (pairs of a row's
 // neighbour groups of `group` variables): `rows` lists the rows by falling work, about d deg^2,
 // so that the uneven tasks are started largest first, and `tasks` is the prefix of their task
-// counts in that order.
+// counts in that order.  From these it chooses the level's route (max_dim: the largest
+// cardinality; planes: the planes before each variable).
 __global__ void __launch_bounds__(1024) disc_plan_kernel(const int *__restrict__ adj, int p, int L, int group,
+                                                         int max_dim, long long n, const int *__restrict__ planes,
                                                          const uint8_t *__restrict__ dims, long long *__restrict__ w,
                                                          long long *__restrict__ prefix, long long *__restrict__ tasks,
                                                          int *__restrict__ rows, DevState *st) {
     extern __shared__ long long s_key[];
+    __shared__ unsigned long long s_task, s_passes;
     if (st->done) return;
+    if (threadIdx.x == 0) s_task = s_passes = 0ull;
     unsigned long long edges = 0;
     for (int r = threadIdx.x; r < p; r += blockDim.x) {
         const int deg = adj[(size_t)r * p];
@@ -507,11 +533,31 @@ __global__ void __launch_bounds__(1024) disc_plan_kernel(const int *__restrict__
     __syncthreads();
     if (threadIdx.x == 0) st->tests_full[L] = (unsigned long long)prefix[p];
     if (group <= 0) return;
+    const float mean = (float)planes[p] / (float)p;  // planes of a variable
+    const long long words = (n + 2047) / 2048;       // passes of 64 words over the samples
+    unsigned long long longest = 0ull, passes = 0ull;
     for (int r = threadIdx.x; r < p; r += blockDim.x) {
         const long long deg = adj[(size_t)r * p];
         s_key[r] = w[r] > 0 ? deg * deg * dims[r] : 0;
+        if (w[r] > 0) {  // blocks of 4 x 4 planes of two groups, for every value of the row's variable but the last
+            const long long side = (long long)ceilf(0.25f * mean * (float)min((long long)group, deg));
+            const long long ng = (deg + group - 1) / group, task = side * side * (dims[r] - 1) * words;
+            longest = max(longest, (unsigned long long)task);
+            passes += (unsigned long long)(task * (ng * (ng + 1) / 2));
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        longest = max(longest, __shfl_xor_sync(GCSL_FULL_MASK, longest, o));
+        passes += __shfl_xor_sync(GCSL_FULL_MASK, passes, o);
+    }
+    if ((threadIdx.x & 31) == 0 && passes) {
+        atomicMax(&s_task, longest);
+        atomicAdd(&s_passes, passes);
     }
     __syncthreads();
+    if (threadIdx.x == 0)
+        st->disc_route = disc_level1_route((float)prefix[p], (float)s_task, (float)s_passes, max_dim, mean, (float)n);
     for (int r = threadIdx.x; r < p; r += blockDim.x) {
         const long long key = s_key[r];
         int rank = 0;
@@ -626,8 +672,12 @@ cudaError_t launch_disc_tests(const DiscLevelArgs &A, int num_sms, cudaStream_t 
         per_sm = 1;
     const int cap = blocks_per_sm_cap();  // room left on every SM for concurrent solves
     if (cap > 0 && per_sm > cap) per_sm = cap;
-    disc_test_kernel<<<num_sms * per_sm, threads, smem, s>>>(A);
     note_launch(1);
+    // behind the bit-plane kernel it often has nothing to do: its launch overlaps that one's end
+    if (A.routed)
+        return note_error("disc_test_kernel launch", launch_pdl(disc_test_kernel, dim3((unsigned)(num_sms * per_sm)),
+                                                                dim3((unsigned)threads), smem, s, A));
+    disc_test_kernel<<<num_sms * per_sm, threads, smem, s>>>(A);
     return note_error("disc_test_kernel launch", cudaGetLastError());
 }
 
@@ -640,10 +690,11 @@ cudaError_t launch_disc_validate(const uint8_t *data, long long ld, long long n,
 }
 
 // group: neighbours per group of the bit-plane path's level 1 (0: no tasks).
-cudaError_t launch_disc_plan(const int *adj, int p, int L, int group, const uint8_t *dims, long long *w,
-                             long long *prefix, long long *tasks, int *rows, DevState *st, cudaStream_t s) {
+cudaError_t launch_disc_plan(const int *adj, int p, int L, int group, int max_dim, long long n, const int *planes,
+                             const uint8_t *dims, long long *w, long long *prefix, long long *tasks, int *rows,
+                             DevState *st, cudaStream_t s) {
     const size_t smem = group > 0 ? (size_t)p * sizeof(long long) : 0;  // p <= 4096 with groups
-    disc_plan_kernel<<<1, 1024, smem, s>>>(adj, p, L, group, dims, w, prefix, tasks, rows, st);
+    disc_plan_kernel<<<1, 1024, smem, s>>>(adj, p, L, group, max_dim, n, planes, dims, w, prefix, tasks, rows, st);
     note_launch(1);
     return cudaGetLastError();
 }

@@ -43,8 +43,9 @@ def test_sets_of_a_repeated_solve(cuda):
     a, b = rng.integers(0, 2, n), rng.integers(0, 2, n)
     w = (rng.random(n) < 0.35 + 0.3 * b + 0.07 * a).astype(int)
     w = np.where(w == 1, 1 + (rng.random(n) < 0.2 + 0.6 * a), 0)
-    codes = np.stack([a, b, w]).astype(np.uint8)
-    merged = oracle_discrete(np.minimum(codes, 1), np.full(3, 2, np.uint8), 0.05, 1)
+    # constant columns beside them: enough variables for the bit planes
+    codes = np.concatenate([np.stack([a, b, w]), np.zeros((37, n), np.int64)]).astype(np.uint8)
+    merged = oracle_discrete(np.minimum(codes, 1), np.minimum(codes.max(1) + 1, 2).astype(np.uint8), 0.05, 1)
     assert merged[0][0, 2] == 0 and merged[1][0, 2, 0] == 1  # what the first attempt finds
     dims = codes.max(1).astype(np.uint8) + 1
     rc, got = run_entry(cuda, codes, dims, 0.05, 1, 2)
