@@ -250,6 +250,7 @@ enum {
     GCSL_DCHECK_POSITION = 2,  // an unranked position outside [1, K]
     GCSL_DCHECK_SET = 3,       // a conditioning variable outside [0, p), equal to v_i / v_j, or unsorted
     GCSL_DCHECK_DEGREE = 4,    // a compacted degree above p - 1
+    GCSL_DCHECK_CELL = 5,      // a plane, word, value or table cell of the bit-plane path outside its buffer
 };
 __device__ __forceinline__ bool dcheck(DevState *st, bool ok, int site) {
 #if GCSL_DEBUG_CHECKS

@@ -260,7 +260,8 @@ __device__ __forceinline__ int slice_words(long long words, long long blocks, lo
 // resident warps a few times over.
 __global__ void __launch_bounds__(256, 2) disc_pair_counts_kernel(const uint32_t *__restrict__ planes, long long words,
                                                                   const int *__restrict__ off, int p,
-                                                                  uint32_t *__restrict__ counts, int ldc) {
+                                                                  uint32_t *__restrict__ counts, int ldc,
+                                                                  DevState *st) {
     const int lane = threadIdx.x & 31;
     const int S = off[p];
     const long long nb = (S + BP_SIDE - 1) / BP_SIDE;
@@ -283,6 +284,7 @@ __global__ void __launch_bounds__(256, 2) disc_pair_counts_kernel(const uint32_t
             co[i] = (uint32_t)(min((int)(BP_SIDE * c) + i, S - 1) * words);
         }
         const long long w0 = sl * per, w1 = w0 + per < words ? w0 + per : words;
+        if (!dcheck(st, S <= ldc && c < nb && w0 < w1 && (w1 - w0) % BP_ROUND == 0, GCSL_DCHECK_CELL)) continue;
         const uint32_t got = popc_block<false>(planes, ro, co, 0u, (int)w0, (int)(w1 - w0) / BP_ROUND);
         const int x = (int)(BP_SIDE * r) + lane / 4, y = (int)(BP_SIDE * c) + lane % 4;
         if (lane < 16 && x <= y && y < S && got != 0) {
@@ -386,7 +388,12 @@ __global__ void __launch_bounds__(BP_L0_THREADS) disc_level0_kernel(
             while (u > 0 && u * (u + 1) / 2 > t) --u;
             while ((u + 1) * (u + 2) / 2 <= t) ++u;
             const int vi = (int)u, vj = (int)(t - u * (u + 1) / 2);
-            const int x = off[vi], y = off[vj], di = dims[vi], dj = dims[vj], fi = foff[vi], fj = foff[vj];
+            int x = off[vi], y = off[vj], di = dims[vi], dj = dims[vj], fi = foff[vi], fj = foff[vj];
+            if (!dcheck(st, vi < p && min(di, dj) >= 1 && max(di, dj) <= 16 && max(x + di, y + dj) - 1 <= ldc &&
+                                max(fi + di, fj + dj) <= ldf, GCSL_DCHECK_CELL)) {
+                x = y = fi = fj = 0;
+                di = dj = 1;
+            }
             uint32_t *tab = s_tab[gw], *nr = s_nr[gw], *nc = s_nc[gw];
             for (int a = gl; a < di - 1; a += BP_LANES) nr[a] = __ldg(counts + (size_t)(x + a) * (ldc + 1));
             for (int b = gl; b < dj - 1; b += BP_LANES) nc[b] = __ldg(counts + (size_t)(y + b) * (ldc + 1));
@@ -574,11 +581,15 @@ __global__ void __launch_bounds__(BP_L1_THREADS, 512 / BP_L1_THREADS) disc_bits_
         const long long t = work_order(s_task, total, A.order);
         const int ri = upper_row(tasks, p, t), i = rows[ri];
         const int *nbrs = A.adj + (size_t)i * p + 1;
-        const int deg = nbrs[-1], di = A.dims[i];
+        const int deg = nbrs[-1];
+        int di = A.dims[i];
         const int ng = (deg + Ly.vars - 1) / Ly.vars;
         int h = (int)(t - tasks[ri]), g = 0;
         while (h >= ng - g) h -= ng - g, ++g;
         h += g;
+        if (!dcheck(st, g < ng && h < ng && deg < p, GCSL_DCHECK_SET)) g = h = 0;
+        if (!dcheck(st, di >= 1 && di <= max_dim && off[i] + di - 1 <= off[p] && foff[i] + di <= ldf, GCSL_DCHECK_CELL))
+            di = 1;
         // the two groups' variables, planes and values (warps 0 and 1)
         if (warp < 2) {
             const int g0 = (warp ? h : g) * Ly.vars, cntv = min(Ly.vars, deg - g0);
@@ -587,7 +598,10 @@ __global__ void __launch_bounds__(BP_L1_THREADS, 512 / BP_L1_THREADS) disc_bits_
                 const int k = k0 + lane;
                 int v = k < cntv ? nbrs[g0 + k] : 0;
                 if (!dcheck(st, v >= 0 && v < p && (k >= cntv || v != i), GCSL_DCHECK_SET)) v = 0;
-                const int d = k < cntv ? A.dims[v] : 0;
+                int d = k < cntv ? A.dims[v] : 0;
+                if (!dcheck(st, k >= cntv || (d >= 1 && d <= max_dim && off[v] + d - 1 <= off[p] && foff[v] + d <= ldf),
+                            GCSL_DCHECK_CELL))
+                    d = 0;
                 int a = d > 1 ? d - 1 : 0, b = d;
                 const int a1 = a, b1 = b;
 #pragma unroll
@@ -672,10 +686,12 @@ __global__ void __launch_bounds__(BP_L1_THREADS, 512 / BP_L1_THREADS) disc_bits_
                         co[k] = (uint32_t)(s_plane[1][min(BP_SIDE * c + k, nc - 1)] * words);
                     }
                     const int w0 = sl * per, w1 = (int)min((long long)w0 + per, words);
+                    if (!dcheck(st, w0 < w1 && (w1 - w0) % BP_ROUND == 0, GCSL_DCHECK_CELL)) continue;
                     const uint32_t got =
                         popc_block<true>(planes, ro, co, mo + (uint32_t)(a * words), w0, (w1 - w0) / BP_ROUND);
                     const int x = BP_SIDE * r + lane / 4, y = BP_SIDE * c + lane % 4;
-                    if (lane < 16 && x < nr && y < nc)
+                    if (lane < 16 && x < nr && y < nc &&
+                        dcheck(st, s_at[0][x] < fr && s_at[1][y] < fc, GCSL_DCHECK_CELL))
                         atomicAdd(cnt + a * plane_sz + s_at[0][x] * ld + s_at[1][y], got);
                 }
             }
@@ -756,7 +772,11 @@ __global__ void __launch_bounds__(BP_L1_THREADS, 512 / BP_L1_THREADS) disc_bits_
             const TripleTable T = table(x, y, k & 1);
             const int df = (T.di - 1) * (T.du - 1) * T.dw;
             if (A.alpha > 0.0 && df > 0 && pvalue_zero(chi2_floor(T, gl, mask), df)) continue;
-            if (gl == 0) queue[atomicAdd(&s_queued, 1)] = (x << 16) | (y << 1) | (k & 1);
+            if (gl == 0) {
+                const int slot = atomicAdd(&s_queued, 1);
+                if (dcheck(st, x < vr && y < vc && slot < 2 * Ly.vars * Ly.vars, GCSL_DCHECK_CELL))
+                    queue[slot] = (x << 16) | (y << 1) | (k & 1);
+            }
         }
         __syncthreads();
         const int queued = s_queued;
@@ -823,7 +843,7 @@ cudaError_t launch_disc_bits_level0(const DiscBits &b, const DiscLevelArgs &A, i
     disc_planes_kernel<<<cap > 0 ? std::min(items, num_sms * cap) : items, 256, 0, s>>>(A.data, A.ld, A.n, p, A.dims, b.max_dim, chunks, b.planes,
                                                               words, b.card, b.off, b.foff, b.lg, b.counts,
                                                               (long long)ldc * ldc, A.st);
-    disc_pair_counts_kernel<<<num_sms * (cap == 1 ? 1 : 2), 256, 0, s>>>(b.planes, words, b.off, p, b.counts, ldc);
+    disc_pair_counts_kernel<<<num_sms * (cap == 1 ? 1 : 2), 256, 0, s>>>(b.planes, words, b.off, p, b.counts, ldc, A.st);
     const long long pairs = (long long)p * (p + 1) / 2, lb = (pairs + BP_L0_GROUPS - 1) / BP_L0_GROUPS;
     const long long l0_per_sm = cap > 0 ? std::min(16, cap * (256 / BP_L0_THREADS)) : 16;
     disc_level0_kernel<<<(unsigned)std::min(lb, num_sms * l0_per_sm), BP_L0_THREADS, 0, s>>>(
