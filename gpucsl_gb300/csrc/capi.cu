@@ -35,7 +35,7 @@ cudaError_t launch_gauss_level(int L, const double *C, int p, const int *adj, co
 
 size_t orient_workspace_bytes(int p);
 cudaError_t encode_columns(const void *X, int dtype, long long n, int p, long long ld, uint8_t *codes, long long ldc,
-                           uint8_t *dims, void *workspace, cudaStream_t s);
+                           uint8_t *dims, void *workspace, int num_sms, cudaStream_t s);
 size_t encode_workspace_bytes(int p);
 cudaError_t orient_edges(const uint16_t *S, int p, const int *sep, int L, uint8_t *D, void *ws, int num_sms,
                          int *host_word, int *passes, cudaStream_t s);
@@ -81,10 +81,10 @@ cudaError_t corr_tc(const void *X, int dtype, long long n, int p, long long ldx,
 cudaError_t corr_tc_digits(const void *X, int dtype, long long n, int p, long long ldx, void *ws, size_t ws_bytes,
                            int num_sms, cudaStream_t s);
 cudaError_t corr_tc_product(long long n, int p, double *C, void *ws, size_t ws_bytes, int num_sms, cudaStream_t s);
-size_t corr_tc_batch_workspace_bytes(const long long *n, const int *p, int count);
+size_t corr_tc_batch_workspace_bytes(const long long *n, const int *p, int count, int num_sms);
 cudaError_t corr_tc_batch_prepare(const void *const *X, const long long *n, const int *p, const long long *ldx,
                                   double *const *C, float *const *C32, int count, void *ws, size_t ws_bytes,
-                                  long long *stage_totals, cudaStream_t s);
+                                  int num_sms, long long *stage_totals, cudaStream_t s);
 cudaError_t corr_tc_batch_run(void *ws, int count, const long long *stage_totals, int dtype, cudaStream_t s);
 size_t gauss_batch_workspace_bytes(const int *p, int count);
 int gauss_batch_prepare(const gcsl_gauss_instance *in, int count, int max_level, int precision, void *ws,
@@ -1049,7 +1049,7 @@ size_t gcsl_corr_tc_batch_workspace_bytes(const int64_t *n, const int32_t *p, in
         nn[(size_t)k] = n[k];
         pp[(size_t)k] = p[k];
     }
-    return host::corr_tc_batch_workspace_bytes(nn.data(), pp.data(), count);
+    return host::corr_tc_batch_workspace_bytes(nn.data(), pp.data(), count, device_sms());
 }
 
 int gcsl_corr_tc_batch_prepare(const void *const *X, int32_t dtype, const int64_t *n, const int32_t *p,
@@ -1066,12 +1066,12 @@ int gcsl_corr_tc_batch_prepare(const void *const *X, int32_t dtype, const int64_
         pp[(size_t)k] = p[k];
         ll[(size_t)k] = ldx[k];
     }
-    if (workspace_bytes < host::corr_tc_batch_workspace_bytes(nn.data(), pp.data(), count)) return GCSL_ERR_WORKSPACE;
+    if (workspace_bytes < host::corr_tc_batch_workspace_bytes(nn.data(), pp.data(), count, device_sms())) return GCSL_ERR_WORKSPACE;
     long long *w = reinterpret_cast<long long *>(plan->w);
     std::memset(w, 0, sizeof(plan->w));
     const cudaError_t e =
         host::corr_tc_batch_prepare(X, nn.data(), pp.data(), ll.data(), C, C32, count, workspace, workspace_bytes,
-                                    w + 4, static_cast<cudaStream_t>(stream));
+                                    device_sms(), w + 4, static_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return GCSL_ERR_DEVICE;
     w[0] = kCorrPlanMagic;
     w[1] = (long long)reinterpret_cast<uintptr_t>(workspace);
@@ -1143,7 +1143,7 @@ int gcsl_ordinal_encode(const void *X, int32_t dtype, int64_t n, int32_t p, int6
     int *status = static_cast<int *>(workspace);  // the workspace starts with the status word
     HostCtl *hc = host_ctl();
     if (!hc) return GCSL_ERR_DEVICE;
-    cudaError_t e = host::encode_columns(X, dtype, n, p, ld, codes, ldc, dims, workspace, s);
+    cudaError_t e = host::encode_columns(X, dtype, n, p, ld, codes, ldc, dims, workspace, device_sms(), s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(&hc->words[0], status, sizeof(int), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return map_cuda(e);

@@ -1328,21 +1328,21 @@ static size_t batch_header_bytes(int count) {
 // a small batch was twice an SM's share), within bounds that keep a block's fixed cost (about
 // ten steps) small and let the few problems of an exact rerun spread over the SMs.
 // 24 problems: product 642 -> 395 us; the exact rerun of a split batch of 256: 707 -> 474 us.
-static long long batch_split_steps(const long long *n, const int *p, int count) {
+static long long batch_split_steps(const long long *n, const int *p, int count, int num_sms) {
     long long total = 0;
     for (int k = 0; k < count; ++k) {
         const OzDims D = oz_dims(n[k], p[k], 1, 1);
         total += (long long)oz_tiles(D) * (D.n_pad / 16);
     }
-    return std::min(512ll, std::max(128ll, total / (4 * 152)));
+    return std::min(512ll, std::max(128ll, total / (4ll * num_sms)));
 }
 static int batch_splits(long long n, long long split_steps) {
     return (int)std::max(1ll, ((n + 15) / 16 + split_steps - 1) / split_steps);
 }
 
-size_t corr_tc_batch_workspace_bytes(const long long *n, const int *p, int count) {
+size_t corr_tc_batch_workspace_bytes(const long long *n, const int *p, int count, int num_sms) {
     size_t total = batch_header_bytes(count);
-    const long long split_steps = batch_split_steps(n, p, count);
+    const long long split_steps = batch_split_steps(n, p, count, num_sms);
     for (int k = 0; k < count; ++k) {
         OzJob J;
         total += oz_job(J, nullptr, nullptr, n[k], p[k], p[k], 1, batch_splits(n[k], split_steps));
@@ -1352,13 +1352,13 @@ size_t corr_tc_batch_workspace_bytes(const long long *n, const int *p, int count
 
 cudaError_t corr_tc_batch_prepare(const void *const *X, const long long *n, const int *p, const long long *ldx,
                                   double *const *C, float *const *C32, int count, void *ws, size_t ws_bytes,
-                                  long long *stage_totals, cudaStream_t s) {
-    if (ws_bytes < corr_tc_batch_workspace_bytes(n, p, count)) return cudaErrorInvalidValue;
+                                  int num_sms, long long *stage_totals, cudaStream_t s) {
+    if (ws_bytes < corr_tc_batch_workspace_bytes(n, p, count, num_sms)) return cudaErrorInvalidValue;
     std::vector<OzJob> jobs((size_t)count);
     std::vector<long long> off((size_t)OZ_NSTAGES * (count + 1), 0);
     char *base = static_cast<char *>(ws);
     size_t cur = batch_header_bytes(count);
-    const long long split_steps = batch_split_steps(n, p, count);
+    const long long split_steps = batch_split_steps(n, p, count, num_sms);
     for (int k = 0; k < count; ++k) {
         OzJob &J = jobs[(size_t)k];
         cur += oz_job(J, base + cur, X[k], n[k], p[k], ldx[k], 1, batch_splits(n[k], split_steps));

@@ -37,8 +37,7 @@ constexpr int ENC_WORDS = ENC_RANGE / 32;
 // 124; 50000 x 2000 (3648 rows) 509, 401.
 constexpr int ENC_PAD_ROWS = 1024;
 constexpr int ENC_STEP = 64;     // rows per step of a block: 8 warps x 8 loads a thread
-// Row chunks are sized for this many blocks: six of the eight blocks an SM holds.
-constexpr int ENC_BLOCKS = 6 * 152;
+constexpr int ENC_BLOCKS = 6;    // blocks an SM that the row chunks are sized for: six of the eight it holds
 
 // Per-column scratch of the encoder.
 struct EncWs {
@@ -343,15 +342,15 @@ static EncWs enc_ws(void *ws, int p) {
 
 template <typename T>
 static cudaError_t encode_typed(const T *X, long long n, int p, long long ld, uint8_t *codes, long long ldc,
-                                uint8_t *dims, const EncWs &w, cudaStream_t s) {
-    const int strips = (p + 31) / 32;
-    const int init_blocks = std::min((p + 7) / 8, ENC_BLOCKS);
+                                uint8_t *dims, const EncWs &w, int num_sms, cudaStream_t s) {
+    const int strips = (p + 31) / 32, all = ENC_BLOCKS * num_sms;
+    const int init_blocks = std::min((p + 7) / 8, all);
     enc_init_kernel<<<(unsigned)init_blocks, 256, 0, s>>>(n, p, dims, w);
     note_launch(1);
     cudaError_t e = cudaGetLastError();
     if (n == 0 || e != cudaSuccess) return e;
-    // whole steps a tile, about ENC_BLOCKS tiles in all, at most 65535 along the rows
-    const long long want = std::max(1, ENC_BLOCKS / strips);
+    // whole steps a tile, about `all` tiles in all, at most 65535 along the rows
+    const long long want = std::min(65535, std::max(1, all / strips));
     long long rows = (n + want - 1) / want;
     rows = (rows + ENC_STEP - 1) / ENC_STEP * ENC_STEP;
     const dim3 grid((unsigned)strips, (unsigned)((n + rows - 1) / rows));
@@ -367,13 +366,13 @@ static cudaError_t encode_typed(const T *X, long long n, int p, long long ld, ui
 
 // status: the first int of the workspace (cleared here); the caller reads it back.
 cudaError_t encode_columns(const void *X, int dtype, long long n, int p, long long ld, uint8_t *codes, long long ldc,
-                           uint8_t *dims, void *workspace, cudaStream_t s) {
+                           uint8_t *dims, void *workspace, int num_sms, cudaStream_t s) {
     const EncWs w = enc_ws(workspace, p);
     switch (dtype) {
-    case GCSL_DTYPE_I32: return encode_typed(static_cast<const int *>(X), n, p, ld, codes, ldc, dims, w, s);
-    case GCSL_DTYPE_I64: return encode_typed(static_cast<const long long *>(X), n, p, ld, codes, ldc, dims, w, s);
-    case GCSL_DTYPE_U8: return encode_typed(static_cast<const uint8_t *>(X), n, p, ld, codes, ldc, dims, w, s);
-    case GCSL_DTYPE_F64: return encode_typed(static_cast<const double *>(X), n, p, ld, codes, ldc, dims, w, s);
+    case GCSL_DTYPE_I32: return encode_typed(static_cast<const int *>(X), n, p, ld, codes, ldc, dims, w, num_sms, s);
+    case GCSL_DTYPE_I64: return encode_typed(static_cast<const long long *>(X), n, p, ld, codes, ldc, dims, w, num_sms, s);
+    case GCSL_DTYPE_U8: return encode_typed(static_cast<const uint8_t *>(X), n, p, ld, codes, ldc, dims, w, num_sms, s);
+    case GCSL_DTYPE_F64: return encode_typed(static_cast<const double *>(X), n, p, ld, codes, ldc, dims, w, num_sms, s);
     default: return cudaErrorInvalidValue;
     }
 }
