@@ -29,12 +29,12 @@ namespace gcsl {
 
 constexpr int ENC_RANGE = 4096;  // values per column: min .. min + 4095
 constexpr int ENC_WORDS = ENC_RANGE / 32;
-// Tiles of at most this many rows keep the bitmaps (words) and ranks (bytes) of their 32 columns in
-// shared memory at a pitch of 33 words and 36 bytes: loading, ranking and merging them, word by
-// word along a column, is then free of bank conflicts, and the rows' accesses, at random words,
-// share a bank three ways.  At 32 it is the other way round, which pays off over many rows.  Columns
-// over 100 values, int32, 33 against 32: 5000 x 1000 (192 rows) 95, 130 us; 50000 x 200 (448 rows) 94,
-// 124; 50000 x 2000 (3648 rows) 509, 401.
+// Tiles of at most this many rows have the bitmaps (words) and ranks (bytes) of pass 2 in shared
+// memory at a pitch of 33 words and 36 bytes: loading and ranking them, word by word along a
+// column, is then free of bank conflicts, and the rows' look-ups, at random words, share a bank
+// three ways.  At 32 it is the other way round, which pays off over many rows.  Columns over 100
+// values, int32, 33 against 32: 5000 x 1000 (192 rows) 97, 126 us; 50000 x 200 (448 rows) 87, 122;
+// 50000 x 2000 (3648 rows) 509, 401.
 constexpr int ENC_PAD_ROWS = 1024;
 constexpr int ENC_STEP = 64;     // rows per step of a block: 8 warps x 8 loads a thread
 constexpr int ENC_BLOCKS = 6;    // blocks an SM that the row chunks are sized for: six of the eight it holds
@@ -101,14 +101,14 @@ __global__ void __launch_bounds__(256) enc_init_kernel(long long n, int p, uint8
 }
 
 // Pass 1: tile (blockIdx.x: 32 columns, blockIdx.y: rows); lane = column.
-template <typename T, bool PAD>
+template <typename T>
 __global__ void __launch_bounds__(256) enc_scan_kernel(const T *__restrict__ X, long long n, int p, long long ld,
                                                       int rows, EncWs w) {
     using V = typename EncInt<T>::type;
     __shared__ V smin[8][32], smax[8][32];
     __shared__ unsigned long long smask[8][32];
     __shared__ int sbad[32];
-    __shared__ unsigned bits[ENC_WORDS][PAD ? 33 : 32];
+    __shared__ unsigned bits[ENC_WORDS][32];
     pdl_trigger();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int j = blockIdx.x * 32 + lane;
@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(256) enc_scan_kernel(const T *__restrict__ X, 
         }
     }
     if (!any_wide) return;
-    for (int k = threadIdx.x; k < (PAD ? 33 : 32) * ENC_WORDS; k += blockDim.x) (&bits[0][0])[k] = 0u;
+    for (int k = threadIdx.x; k < 32 * ENC_WORDS; k += blockDim.x) (&bits[0][0])[k] = 0u;
     __syncthreads();
     if (j < p) {
         for (long long t = t0 + warp; t < t1; t += 8) {
@@ -180,17 +180,9 @@ __global__ void __launch_bounds__(256) enc_scan_kernel(const T *__restrict__ X, 
         }
     }
     __syncthreads();
-    if constexpr (PAD) {
-        for (int q = warp; q < ENC_WORDS; q += 8) {  // lane = one of 32 words of a column
-            const int c = q / (ENC_WORDS / 32), wd = q % (ENC_WORDS / 32) * 32 + lane, jc = blockIdx.x * 32 + c;
-            const unsigned b = bits[wd][c];
-            if (b != 0u && jc < p) atomicOr(w.bits + (size_t)jc * ENC_WORDS + wd, b);
-        }
-    } else {
-        for (int wd = warp; wd < ENC_WORDS; wd += 8) {
-            const unsigned b = bits[wd][lane];
-            if (b != 0u && j < p) atomicOr(w.bits + (size_t)j * ENC_WORDS + wd, b);
-        }
+    for (int wd = warp; wd < ENC_WORDS; wd += 8) {
+        const unsigned b = bits[wd][lane];
+        if (b != 0u && j < p) atomicOr(w.bits + (size_t)j * ENC_WORDS + wd, b);
     }
 }
 
@@ -355,8 +347,7 @@ static cudaError_t encode_typed(const T *X, long long n, int p, long long ld, ui
     rows = (rows + ENC_STEP - 1) / ENC_STEP * ENC_STEP;
     const dim3 grid((unsigned)strips, (unsigned)((n + rows - 1) / rows));
     const bool pad = rows <= ENC_PAD_ROWS;
-    e = launch_pdl(pad ? enc_scan_kernel<T, true> : enc_scan_kernel<T, false>, grid, dim3(256), 0, s, X, n, p, ld,
-                   (int)rows, w);
+    e = launch_pdl(enc_scan_kernel<T>, grid, dim3(256), 0, s, X, n, p, ld, (int)rows, w);
     if (e == cudaSuccess)
         e = launch_pdl(pad ? enc_codes_kernel<T, true> : enc_codes_kernel<T, false>, grid, dim3(256), 0, s, X, n, p, ld,
                        (int)rows, codes, ldc, dims, w);

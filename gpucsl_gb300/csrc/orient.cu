@@ -69,27 +69,36 @@ __device__ __forceinline__ bool arc(const uint8_t *D, int p, int a, int b) {
     return __ldcg(D + (size_t)a * p + b) != 0;
 }
 
+// A warp's rows first, first + step, ..; with more warps than rows several share one and take
+// turns in its neighbours.
+struct RowShare {
+    int first, step, part, share;
+    __device__ __forceinline__ RowShare(int p, int warp, int warps) {
+        share = warps > p ? warps / p : 1;
+        step = warps / share;
+        part = warp / step;
+        first = part < share ? warp - part * step : p;  // the last few warps: no rows
+    }
+};
+
 // f(a, b, list of a, degree of a, lane of the group, group mask) for every directed pair
-// (a, b) of adjacent vertices: eight lanes per neighbour b; warp per row a, or with more warps
-// than rows several per row, which take turns in its neighbours.
+// (a, b) of adjacent vertices: eight lanes per neighbour b.
 template <typename F>
-__device__ __forceinline__ void for_edges(const int *adj, int p, int warp, int warps, F f) {
+__device__ __forceinline__ void for_edges(const int *adj, int p, const RowShare &rs, F f) {
     const int lane = threadIdx.x & 31, sub = lane & 7;
     const unsigned group = 0xffu << (lane & 24);
-    const int share = warps > p ? warps / p : 1, rows = warps / share, part = warp / rows;
-    if (part >= share) return;
-    for (int a = warp - part * rows; a < p; a += rows) {
+    for (int a = rs.first; a < p; a += rs.step) {
         const int *ra = adj + (size_t)a * p;
         const int da = __ldcg(ra);
-        for (int t = 4 * part + (lane >> 3); t < da; t += 4 * share) f(a, __ldcg(ra + 1 + t), ra, da, sub, group);
+        for (int t = 4 * rs.part + (lane >> 3); t < da; t += 4 * rs.share) f(a, __ldcg(ra + 1 + t), ra, da, sub, group);
     }
 }
 
 // P[a][b] for every skeleton edge: some neighbour v != a of b, non-adjacent to a, with b
 // in neither sepset(a, v) nor sepset(v, a).
 __device__ __forceinline__ void vstruct_flags(const uint16_t *__restrict__ S, const int *adj, int p,
-                                              const int *__restrict__ sep, int L, uint8_t *P, int warp, int warps) {
-    for_edges(adj, p, warp, warps, [&](int a, int b, const int *, int, int sub, unsigned group) {
+                                              const int *__restrict__ sep, int L, uint8_t *P, const RowShare &rs) {
+    for_edges(adj, p, rs, [&](int a, int b, const int *, int, int sub, unsigned group) {
         const int *rb = adj + (size_t)b * p;
         const int db = __ldcg(rb);
         bool hit = false;
@@ -128,10 +137,10 @@ __device__ __forceinline__ void fire_edge(unsigned long long *key, int p, int fr
 
 // R1 on snapshot D: v1 -> v2 (directed only), v2 - v3 undirected, v1 and v3
 // non-adjacent: orient v2 -> v3.  Earliest key per edge.  True if the thread fired one.
-__device__ __forceinline__ bool rule1(const int *adj, int p, const uint8_t *D, unsigned long long *key, int warp,
-                                      int warps) {
+__device__ __forceinline__ bool rule1(const int *adj, int p, const uint8_t *D, unsigned long long *key,
+                                      const RowShare &rs) {
     bool fired = false;
-    for_edges(adj, p, warp, warps, [&](int v1, int v2, const int *, int, int sub, unsigned) {
+    for_edges(adj, p, rs, [&](int v1, int v2, const int *, int, int sub, unsigned) {
         const int *r2 = adj + (size_t)v2 * p;
         const int d2 = __ldcg(r2);
         if (!arc(D, p, v1, v2) || arc(D, p, v2, v1)) return;
@@ -150,10 +159,10 @@ __device__ __forceinline__ bool rule1(const int *adj, int p, const uint8_t *D, u
 // v1 - v2 undirected in D: R2 some v3 with v1 -> v3 -> v2 directed only; R3 two non-adjacent
 // v3, v4 with v1 - v3 -> v2, v1 - v4 -> v2.  Orient v1 -> v2, latest key per edge.
 template <int RULE>
-__device__ __forceinline__ bool rule23(const int *adj, int p, const uint8_t *D, unsigned long long *key, int warp,
-                                       int warps) {
+__device__ __forceinline__ bool rule23(const int *adj, int p, const uint8_t *D, unsigned long long *key,
+                                       const RowShare &rs) {
     bool fired = false;
-    for_edges(adj, p, warp, warps, [&](int v1, int v2, const int *r1, int d1, int sub, unsigned group) {
+    for_edges(adj, p, rs, [&](int v1, int v2, const int *r1, int d1, int sub, unsigned group) {
         if (!arc(D, p, v1, v2) || !arc(D, p, v2, v1)) return;
         bool fire = false;
         for (int k0 = 0; k0 < d1 && !fire; k0 += 8) {
@@ -254,6 +263,7 @@ __global__ void __launch_bounds__(256, 1) orient_kernel(const uint16_t *__restri
     const int lane = threadIdx.x & 31;
     const long long pp = (long long)p * p, tid = (long long)blockIdx.x * blockDim.x + threadIdx.x,
                     threads = (long long)gridDim.x * blockDim.x;
+    const RowShare rs(p, warp, warps);
     unsigned phase = 0;
     bool fired;
     const long long vec = (reinterpret_cast<uintptr_t>(D) & 15u) == 0 ? pp / 16 : 0;
@@ -267,7 +277,7 @@ __global__ void __launch_bounds__(256, 1) orient_kernel(const uint16_t *__restri
     if (lane == 0 && work != 0ull) atomicAdd(&ctl->work, work);
     if (!or_barrier(ctl, ++phase, false, &fired)) return;
     if (__ldcg(&ctl->work) > OR_MAX_WORK) return;  // (every block alike)
-    vstruct_flags(S, adj, p, sep, L, P, warp, warps);
+    vstruct_flags(S, adj, p, sep, L, P, rs);
     if (!or_barrier(ctl, ++phase, false, &fired)) return;
     vstruct_apply(adj, p, P, D, key, warp, warps);
     if (!or_barrier(ctl, ++phase, false, &fired)) return;
@@ -275,9 +285,9 @@ __global__ void __launch_bounds__(256, 1) orient_kernel(const uint16_t *__restri
     for (int n = 1;; ++n) {
         bool changed = false;
         for (int rule = 1; rule <= 3; ++rule) {
-            const bool f = rule == 1   ? rule1(adj, p, D, key, warp, warps)
-                           : rule == 2 ? rule23<2>(adj, p, D, key, warp, warps)
-                                       : rule23<3>(adj, p, D, key, warp, warps);
+            const bool f = rule == 1   ? rule1(adj, p, D, key, rs)
+                           : rule == 2 ? rule23<2>(adj, p, D, key, rs)
+                                       : rule23<3>(adj, p, D, key, rs);
             if (!or_barrier(ctl, ++phase, f, &fired)) return;
             if (!fired) continue;
             changed = true;
@@ -301,14 +311,15 @@ __global__ void __launch_bounds__(256) orient_step_kernel(const uint16_t *__rest
                                                          uint8_t *P, uint8_t *D, unsigned long long *key, OrCtl *ctl,
                                                          int step) {
     const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), warps = (int)(gridDim.x * blockDim.x) >> 5;
+    const RowShare rs(p, warp, warps);
     bool fired = false;
     switch (step) {
-    case 0: vstruct_flags(S, adj, p, sep, L, P, warp, warps); break;
+    case 0: vstruct_flags(S, adj, p, sep, L, P, rs); break;
     case 1: vstruct_apply(adj, p, P, D, key, warp, warps); break;
-    case 2: fired = rule1(adj, p, D, key, warp, warps); break;
+    case 2: fired = rule1(adj, p, D, key, rs); break;
     case 3: rule_apply(adj, p, D, key, false, warp, warps); break;
-    case 4: fired = rule23<2>(adj, p, D, key, warp, warps); break;
-    case 6: fired = rule23<3>(adj, p, D, key, warp, warps); break;
+    case 4: fired = rule23<2>(adj, p, D, key, rs); break;
+    case 6: fired = rule23<3>(adj, p, D, key, rs); break;
     default: rule_apply(adj, p, D, key, true, warp, warps); break;  // 5, 7
     }
     if (fired) ctl->changed = 1;
