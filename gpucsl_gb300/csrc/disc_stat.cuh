@@ -177,6 +177,24 @@ __device__ inline double pchisq_tab_warp(double x, long long df, const double *_
     return c * y + s;
 }
 
+// The p-value jumps where the published formulation changes branch: at chi^2 = 4 and 36 (pieces
+// of the normal tail) and 40 (the two series, their first term).  chi^2 of few samples is a small
+// fraction and may lie on a jump exactly, or the p-value on alpha; the last bit would then decide.
+// Such a test is evaluated once more in the published order (chi^2 cell by cell, pchisq_dev), by
+// one thread.  (A term's cut at exponent -20 is met by chance only: the exponent has a logarithm.)
+//
+// On it: the 32 bits of two doubles from the fifth-last exponent bit on differ by at most one, a
+// window of at least 2^-28 relative, above the difference of the two evaluations (below 1e-9 up to
+// 2^32 samples) and met by chance once in millions of tests.
+__device__ __forceinline__ unsigned tie_bits(double x) {
+    return __funnelshift_l((unsigned)__double2loint(x), (unsigned)__double2hiint(x), 8);
+}
+__device__ __forceinline__ bool pvalue_tie(double chi2, double pv, double alpha) {
+    const unsigned k = tie_bits(chi2);  // 4, 36, 40: from one step below
+    return (k - 0x0fffffffu <= 1u) | (k - 0x41ffffffu <= 1u) | (k - 0x43ffffffu <= 1u) |
+           (tie_bits(pv) - tie_bits(alpha) + 1u <= 2u);
+}
+
 // A cell's term of a lower bound of chi^2 in FP32: e = N_a N_b / N_s and d = N - e carry
 // relative errors of a few 2^-24 of N + e, taken off |d|.  The error of a sum of these terms
 // and of its quotients is far inside a factor 0.999, which the caller applies.

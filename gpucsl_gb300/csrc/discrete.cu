@@ -264,6 +264,14 @@ __device__ double table_chi2(const uint32_t *sm_tab, int dim_s, int di, int dj, 
     return chi;
 }
 
+// P-value of the counted table in the published order, by one thread (tests on a jump of the
+// p-value).
+__device__ __noinline__ double table_pvalue_ordered(const uint32_t *sm_tab, int dim_s, int di, int dj) {
+    double chi = 0.0;
+    for (int s = 0; s < dim_s; ++s) chi = __dadd_rn(chi, stratum_chi2(sm_tab + (size_t)s * di * dj, di, dj));
+    return pchisq_dev(chi, (long long)(di - 1) * (long long)(dj - 1) * (long long)dim_s);
+}
+
 // Per-test header prepared by thread 0: table geometry and replica count.
 __device__ __forceinline__ bool table_geometry(const uint8_t *dims, const int *S, int *mult, int L, int vi, int vj,
                                                int table_cap, int part_cap, int &dim_s, int &di, int &dj,
@@ -382,6 +390,7 @@ __global__ void __launch_bounds__(DISC_THREADS) disc_test_kernel(DiscLevelArgs A
         if (!zero && tid < 32) {  // warp 0: the p-value's series split over the lanes
             const long long df = (long long)(di - 1) * (long long)(dj - 1) * (long long)dim_s;
             pv = pchisq_tab_warp(chi, df, A.lg);
+            if (tid == 0 && df > 0 && pvalue_tie(chi, pv, A.alpha)) pv = table_pvalue_ordered(sm_tab, dim_s, di, dj);
         }
         if (tid == 0) {
             const int lo = vi < vj ? vi : vj, hi = vi < vj ? vj : vi;

@@ -20,7 +20,7 @@ def independent_codes(p, n, card, seed):
     return codes, np.full(p, card, np.uint8)
 
 
-def solve(torch, codes, dims, level, general):
+def solve(torch, codes, dims, level, general, alpha=0.05):
     from gpucsl_gb300 import _lib, engine
 
     p, n = codes.shape
@@ -28,7 +28,7 @@ def solve(torch, codes, dims, level, general):
     if general:  # no room for the planes
         s.workspace = s.workspace[:int(_lib.lib().gcsl_disc_workspace_bytes(p, n, level, 1))]
     s.load(codes, dims)
-    st = s.run(0.05)
+    st = s.run(alpha)
     return (*s.to_host(), st)
 
 
